@@ -1149,6 +1149,11 @@ int gemm_sub_simt_f32(fp_ctx* c, const float* A, const float* B, float* C, int64
 // then the per-block substitutions and updates (k_strip). Columns are split between the
 // streams so that no element is written by both at once.
 constexpr int kOuterNB = kOuterPanel;
+// Below this many rows the digits' two launches and a tile's latency (35 us)
+// cost what the INT8 update saves: the factorisation of 1,840 unknowns took
+// 3.47 ms with the FP64 tensor path and 3.59 ms with the digits, of 6,300
+// 16.6 and 14.8 ms, of 12,000 58.8 and 43.1 ms.
+constexpr int64_t kI8Rows = 2048;
 
 template <class T>
 int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cert) {
@@ -1182,11 +1187,27 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
     FP_CUDA_TRY(c->err, cudaGetLastError());
     return FP_OK;
   };
+  // FP64: panels with kI8Rows rows below them update on the INT8 tensor cores
+  // (fp_i8.cu) unless a variant of FP_TUNE_FP64_DMMA is asked for; a panel
+  // with columns right of it is whole
+  bool i8 = false;
+  if (sizeof(T) == 8 && c->fp64_dmma == 6 && n >= kOuterNB + kI8Rows &&
+      ((reinterpret_cast<uintptr_t>(A) | (uintptr_t)(lda * 8)) & 15) == 0) {
+    if (int rc = i8_scratch(c, n)) return rc;
+    i8 = true;
+  }
   c->trace.base = tr_event(c);
   // stream2 starts after everything already queued on c->stream
   FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
   FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream2, c->ev_rest, 0));
   for (int64_t K0 = 0; K0 < n; K0 += kOuterNB) {
+    const int set = (int)((K0 / kOuterNB) & 1);
+    // columns [c0, c1) right of the panel -= L21 U12
+    auto update = [&](int64_t kend, int64_t c0, int64_t c1) -> int {
+      if constexpr (sizeof(T) == 8)
+        if (i8 && n - kend >= kI8Rows) return i8_gemm_sub(c, set, at(K0, c0), at(kend, c0), lda, n - kend, c0 - kend, c1 - c0);
+      return gemm_sub<T>(c, at(kend, K0), at(K0, c0), at(kend, c0), lda, n - kend, c1 - c0, (int)(kend - K0));
+    };
     const int64_t kend = std::min<int64_t>(K0 + kOuterNB, n);
     const int64_t knext = std::min<int64_t>(kend + kOuterNB, n);   // next panel: columns [kend, knext)
     // (1) factor the panel's columns, full height
@@ -1228,14 +1249,15 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
     }
+    if constexpr (sizeof(T) == 8)
+      if (i8 && n - kend >= kI8Rows)
+        if (int rc = i8_slice_rows(c, set, at(kend, K0), lda, n - kend)) return rc;
     FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_panel, c->stream));
     // (2) the next panel's columns: P's swaps and U12 rows, then their update
     if (knext > kend) {
       FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream, c->ev_rest, 0));
       if (int rc = strip(K0, (int)(kend - K0), 0, 0, kend, knext)) return rc;
-      if (int rc = gemm_sub<T>(c, at(kend, K0), at(K0, kend), at(kend, kend), lda, n - kend, knext - kend,
-                               (int)(kend - K0)))
-        return rc;
+      if (int rc = update(kend, kend, knext)) return rc;
     }
     // (3) on stream2: swaps left of P, U12 rows beyond the next panel, their update
     {
@@ -1243,9 +1265,7 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
       FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream, c->ev_panel, 0));
       if (int rc = strip(K0, (int)(kend - K0), 0, K0, knext, n)) return rc;
       if (n > knext)
-        if (int rc = gemm_sub<T>(c, at(kend, K0), at(K0, knext), at(kend, knext), lda, n - kend, n - knext,
-                                 (int)(kend - K0)))
-          return rc;
+        if (int rc = update(kend, knext, n)) return rc;
       FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
     }
   }
