@@ -176,6 +176,8 @@ int fp_ctx_create(int device, fp_ctx** out) {
       cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
       cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess || cudaMalloc(&c->d_cert, sizeof(float)) != cudaSuccess ||
       cudaMalloc(&c->d_ticket, sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc(&c->d_p64, 8 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMemset(c->d_p64, 0, 8 * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->d_ticket, 0, sizeof(unsigned)) != cudaSuccess) {
     delete c;
     return FP_ECUDA;
@@ -195,7 +197,7 @@ int fp_ctx_destroy(fp_ctx* c) {
   free_matrices(c);
   post_free(c);
   dfree(c->d_panels); dfree(c->d_src); dfree(c->d_tgt); dfree(c->d_wake);
-  dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket);
+  dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket); dfree(c->d_p64);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->ktimer.pool) cudaEventDestroy(e);

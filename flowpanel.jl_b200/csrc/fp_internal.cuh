@@ -93,6 +93,8 @@ struct fp_ctx {
   unsigned long long* d_mbox = nullptr; // per 128-row block, 128 (epoch, FP32 value) words of the single-RHS sweep
   unsigned trs_epoch = 0;               // epoch of the last sweep launched
   float* d_cert = nullptr;              // max |L| certificate
+  unsigned* d_p64 = nullptr;            // FP64 panel: CTA ticket, then the blocks' flags (both only grow)
+  unsigned p64_ticket = 0, p64_flag = 0;   // their values before the next launch
   unsigned* d_ticket = nullptr;         // ticket of the factorisation's block launches (zero between launches)
   double* d_dinv64 = nullptr;           // inverses of the FP64 diagonal blocks
   float* d_dinv32 = nullptr;            // inverses of the FP32 diagonal blocks
@@ -235,6 +237,11 @@ int launch_rhs(fp_ctx* c, const double* d_U, int64_t k);
 // dense linear algebra (fp_lu.cu)
 template <class T>
 int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cert_max_L);
+template <>   // fp_lu64.cu
+int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipiv, float* cert_max_L);
+// C (m x nn) -= A (m x kk) B (kk x nn) on the FP64 tensor path, blocks of one
+// column-major matrix (16-byte aligned, lda even)
+int gemm_sub_f64(fp_ctx* c, const double* A, const double* B, double* C, int64_t lda, int64_t m, int64_t nn, int kk);
 template <class T>
 int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv, T* B,
              int64_t ldb, int64_t k, bool transpose);

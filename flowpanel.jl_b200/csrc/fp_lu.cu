@@ -1,4 +1,6 @@
-// Dense LU factorisation and triangular solves on sm_100a.
+// Dense LU factorisation (pivoted FP32) and triangular solves on sm_100a; the
+// FP64 factorisation is fp_lu64.cu, which shares the solves and the FP64
+// products of this file.
 //
 // Blocked right-looking LU with partial pivoting inside each NB x NB diagonal
 // block (the search runs over the rows of the block). After the block is
@@ -14,9 +16,8 @@
 // those holding the next block's rows, factors the next diagonal block. After
 // the panel's blocks, (3) k_pfix writes U12 = M' A12 and the row swaps left of
 // each block. Columns outside the panel get the panel's swaps and U12 from
-// k_strip and the trailing update from a GEMM (SIMT FP64, or the 3xTF32
-// tcgen05 kernel of fp_tc.cu for the FP32 factors), on two streams (see
-// lu_factor).
+// k_strip and the trailing update from a GEMM (the 3xTF32 tcgen05 kernel of
+// fp_tc.cu), on two streams (see lu_factor).
 //
 // Triangular solves run in one persistent kernel per sweep: CTAs take row
 // blocks by ticket (atomic counter), wait (bounded) for the blocks they depend
@@ -125,14 +126,6 @@ template <> struct PivKey<float> {
     lo = 0u;
   }
 };
-template <> struct PivKey<double> {
-  __device__ static void of(double v, bool used, unsigned& hi, unsigned& lo) {
-    const unsigned long long b = used ? 0ull : (unsigned long long)__double_as_longlong(fabs(v)) + 1ull;
-    hi = (unsigned)(b >> 32);
-    lo = (unsigned)b;
-  }
-};
-
 // shared workspace of diag_factor: pcand[2][4][NB], S / Lsh [NB][RP],
 // cand[2][4] (uint4), lpiv[NB], rowat[NB]
 template <class T> __host__ __device__ constexpr int diag_ws_bytes() {
@@ -141,7 +134,6 @@ template <class T> __host__ __device__ constexpr int diag_ws_bytes() {
 
 template <class T> __device__ __forceinline__ T rcp_rn(T x);
 template <> __device__ __forceinline__ float rcp_rn<float>(float x) { return __frcp_rn(x); }
-template <> __device__ __forceinline__ double rcp_rn<double>(double x) { return __drcp_rn(x); }
 
 // The 128 threads of the calling CTA factor the diagonal block at k (k_diag;
 // k_blk runs it for the next block once that block's rows are final). A is
@@ -1051,70 +1043,61 @@ k_gemm_sub_dmma(const double* __restrict__ Am, const double* __restrict__ Bm, do
     }
 }
 
-// C (m x nn) -= A (m x kk) B (kk x nn); all three are sub-blocks of one
-// column-major matrix with leading dimension lda.
-template <class T>
-static int gemm_sub(fp_ctx* c, const T* Am, const T* Bm, T* Cm, int64_t lda, int64_t m, int64_t nn,
-                    int kk) {
+int gemm_sub_f64(fp_ctx* c, const double* Am, const double* Bm, double* Cm, int64_t lda, int64_t m, int64_t nn,
+                 int kk) {
   if (m <= 0 || nn <= 0 || kk <= 0) return FP_OK;
-  if constexpr (sizeof(T) == 4) {
-    if (tc_gemm_sub_f32(c, (const float*)Am, (const float*)Bm, (float*)Cm, lda, m, nn, kk)) return FP_OK;
-    return gemm_sub_simt_f32(c, (const float*)Am, (const float*)Bm, (float*)Cm, lda, m, nn, kk);
+  const int slot = kt_begin(c);
+  TraceScope tr(c, TR_GEMM_SIMT);
+  if (c->fp64_dmma) {
+    static SmemAttr attr8, attr16, attr32, attr32k, attr2c, attr2k;
+    constexpr int sm16 = (int)dm::smem<16, 3>(), sm32 = (int)dm::smem<32, 3>();
+    FP_CUDA_TRY(c->err, attr8.ensure(k_gemm_sub_dmma<256, 8, 4>, sm16));
+    FP_CUDA_TRY(c->err, attr16.ensure(k_gemm_sub_dmma<512, 4, 4>, sm16));
+    FP_CUDA_TRY(c->err, attr32.ensure(k_gemm_sub_dmma<1024, 4, 2>, sm16));
+    FP_CUDA_TRY(c->err, attr32k.ensure(k_gemm_sub_dmma<1024, 4, 2, 32, 3>, sm32));
+    constexpr int sm64 = (int)dm::smem<16, 3, 64>();
+    FP_CUDA_TRY(c->err, attr2c.ensure(k_gemm_sub_dmma<512, 4, 2, 16, 3, 64, 2>, sm64));
+    constexpr int sm64k = (int)dm::smem<32, 2, 64>();
+    FP_CUDA_TRY(c->err, attr2k.ensure(k_gemm_sub_dmma<512, 4, 2, 32, 2, 64, 2>, sm64k));
+    dim3 g((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 127) / 128));
+    const double* Ad = (const double*)Am;
+    const double* Bd = (const double*)Bm;
+    double* Cd = (double*)Cm;
+    if (c->fp64_dmma == 6) {   // 128 x 64 tiles, two CTAs an SM, 32-deep K slices in 2 stages
+      dim3 g2((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 63) / 64));
+      k_gemm_sub_dmma<512, 4, 2, 32, 2, 64, 2><<<g2, 512, sm64k, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
+    } else if (c->fp64_dmma == 5) {   // 128 x 64 tiles, two CTAs an SM
+      dim3 g2((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 63) / 64));
+      k_gemm_sub_dmma<512, 4, 2, 16, 3, 64, 2><<<g2, 512, sm64, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
+    } else if (c->fp64_dmma == 4)
+      k_gemm_sub_dmma<1024, 4, 2, 32, 3><<<g, 1024, sm32, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
+    else if (c->fp64_dmma == 3)
+      k_gemm_sub_dmma<1024, 4, 2><<<g, 1024, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
+    else if (c->fp64_dmma == 2)
+      k_gemm_sub_dmma<512, 4, 4><<<g, 512, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
+    else
+      k_gemm_sub_dmma<256, 8, 4><<<g, 256, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
   } else {
-    // cp.async moves 16-byte pieces: the blocks' row offsets and lda must keep them aligned
-    const uintptr_t mis = (reinterpret_cast<uintptr_t>(Am) | reinterpret_cast<uintptr_t>(Bm) |
-                           (uintptr_t)(lda * sizeof(T))) & 15;
-    const int slot = kt_begin(c);
-    TraceScope tr(c, TR_GEMM_SIMT);
-    if (mis == 0 && c->fp64_dmma) {
-      static SmemAttr attr8, attr16, attr32, attr32k, attr2c, attr2k;
-      constexpr int sm16 = (int)dm::smem<16, 3>(), sm32 = (int)dm::smem<32, 3>();
-      FP_CUDA_TRY(c->err, attr8.ensure(k_gemm_sub_dmma<256, 8, 4>, sm16));
-      FP_CUDA_TRY(c->err, attr16.ensure(k_gemm_sub_dmma<512, 4, 4>, sm16));
-      FP_CUDA_TRY(c->err, attr32.ensure(k_gemm_sub_dmma<1024, 4, 2>, sm16));
-      FP_CUDA_TRY(c->err, attr32k.ensure(k_gemm_sub_dmma<1024, 4, 2, 32, 3>, sm32));
-      constexpr int sm64 = (int)dm::smem<16, 3, 64>();
-      FP_CUDA_TRY(c->err, attr2c.ensure(k_gemm_sub_dmma<512, 4, 2, 16, 3, 64, 2>, sm64));
-      constexpr int sm64k = (int)dm::smem<32, 2, 64>();
-      FP_CUDA_TRY(c->err, attr2k.ensure(k_gemm_sub_dmma<512, 4, 2, 32, 2, 64, 2>, sm64k));
-      dim3 g((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 127) / 128));
-      const double* Ad = (const double*)Am;
-      const double* Bd = (const double*)Bm;
-      double* Cd = (double*)Cm;
-      if (c->fp64_dmma == 6) {   // 128 x 64 tiles, two CTAs an SM, 32-deep K slices in 2 stages
-        dim3 g2((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 63) / 64));
-        k_gemm_sub_dmma<512, 4, 2, 32, 2, 64, 2><<<g2, 512, sm64k, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-      } else if (c->fp64_dmma == 5) {   // 128 x 64 tiles, two CTAs an SM
-        dim3 g2((unsigned)((m + dm::BM - 1) / dm::BM), (unsigned)((nn + 63) / 64));
-        k_gemm_sub_dmma<512, 4, 2, 16, 3, 64, 2><<<g2, 512, sm64, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-      } else if (c->fp64_dmma == 4)
-        k_gemm_sub_dmma<1024, 4, 2, 32, 3><<<g, 1024, sm32, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-      else if (c->fp64_dmma == 3)
-        k_gemm_sub_dmma<1024, 4, 2><<<g, 1024, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-      else if (c->fp64_dmma == 2)
-        k_gemm_sub_dmma<512, 4, 4><<<g, 512, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-      else
-        k_gemm_sub_dmma<256, 8, 4><<<g, 256, sm16, c->stream>>>(Ad, Bd, Cd, lda, m, nn, kk, c->tc_prefetch);
-    } else if (mis == 0) {
-      static SmemAttr attr;
-      FP_CUDA_TRY(c->err, attr.ensure(k_gemm_sub_f64, (int)d64::smem()));
-      dim3 g((unsigned)((m + d64::BM - 1) / d64::BM), (unsigned)((nn + d64::BN - 1) / d64::BN));
-      k_gemm_sub_f64<<<g, d64::NT, d64::smem(), c->stream>>>((const double*)Am, (const double*)Bm, (double*)Cm, lda, m,
-                                                             nn, kk);
-    } else {
-      constexpr int BM = 128, BN = 128, BK = 8, TM = 8, TN = 8;
-      constexpr size_t sm = gemm_smem<T, BM, BN, BK, TM, TN>();
-      static SmemAttr attr;
-      FP_CUDA_TRY(c->err, attr.ensure(k_gemm_sub<T, BM, BN, BK, TM, TN>, (int)sm));
-      dim3 g((unsigned)((m + BM - 1) / BM), (unsigned)((nn + BN - 1) / BN));
-      const bool pre = ((reinterpret_cast<uintptr_t>(Cm) | (uintptr_t)(lda * sizeof(T))) & 15) == 0;
-      k_gemm_sub<T, BM, BN, BK, TM, TN><<<g, (BM / TM) * (BN / TN), sm, c->stream>>>(Am, Bm, Cm, lda, m, nn, kk, pre);
-    }
-    kt_end(c, slot, 2.0 * (double)m * (double)nn * (double)kk, (double)m * (double)nn);
-    ++c->nlaunch;
+    static SmemAttr attr;
+    FP_CUDA_TRY(c->err, attr.ensure(k_gemm_sub_f64, (int)d64::smem()));
+    dim3 g((unsigned)((m + d64::BM - 1) / d64::BM), (unsigned)((nn + d64::BN - 1) / d64::BN));
+    k_gemm_sub_f64<<<g, d64::NT, d64::smem(), c->stream>>>((const double*)Am, (const double*)Bm, (double*)Cm, lda, m,
+                                                           nn, kk);
   }
+  kt_end(c, slot, 2.0 * (double)m * (double)nn * (double)kk, (double)m * (double)nn);
+  ++c->nlaunch;
   FP_CUDA_TRY(c->err, cudaGetLastError());
   return FP_OK;
+}
+
+
+// C (m x nn) -= A (m x kk) B (kk x nn); all three are sub-blocks of one
+// column-major matrix with leading dimension lda.
+static int gemm_sub_f32(fp_ctx* c, const float* Am, const float* Bm, float* Cm, int64_t lda, int64_t m, int64_t nn,
+                        int kk) {
+  if (m <= 0 || nn <= 0 || kk <= 0) return FP_OK;
+  if (tc_gemm_sub_f32(c, Am, Bm, Cm, lda, m, nn, kk)) return FP_OK;
+  return gemm_sub_simt_f32(c, Am, Bm, Cm, lda, m, nn, kk);
 }
 
 int gemm_sub_simt_f32(fp_ctx* c, const float* A, const float* B, float* C, int64_t lda, int64_t m, int64_t nn,
@@ -1149,12 +1132,6 @@ int gemm_sub_simt_f32(fp_ctx* c, const float* A, const float* B, float* C, int64
 // then the per-block substitutions and updates (k_strip). Columns are split between the
 // streams so that no element is written by both at once.
 constexpr int kOuterNB = kOuterPanel;
-// Below this many rows the digits' two launches and a tile's latency (35 us)
-// cost what the INT8 update saves: the factorisation of 1,840 unknowns took
-// 3.47 ms with the FP64 tensor path and 3.59 ms with the digits, of 6,300
-// 16.6 and 14.8 ms, of 12,000 58.8 and 43.1 ms.
-constexpr int64_t kI8Rows = 2048;
-
 template <class T>
 int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cert) {
   FP_CUDA_TRY(c->err, cudaMemsetAsync(cert, 0, sizeof(float), c->stream));
@@ -1187,27 +1164,11 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
     FP_CUDA_TRY(c->err, cudaGetLastError());
     return FP_OK;
   };
-  // FP64: panels with kI8Rows rows below them update on the INT8 tensor cores
-  // (fp_i8.cu) unless a variant of FP_TUNE_FP64_DMMA is asked for; a panel
-  // with columns right of it is whole
-  bool i8 = false;
-  if (sizeof(T) == 8 && c->fp64_dmma == 6 && n >= kOuterNB + kI8Rows &&
-      ((reinterpret_cast<uintptr_t>(A) | (uintptr_t)(lda * 8)) & 15) == 0) {
-    if (int rc = i8_scratch(c, n)) return rc;
-    i8 = true;
-  }
   c->trace.base = tr_event(c);
   // stream2 starts after everything already queued on c->stream
   FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
   FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream2, c->ev_rest, 0));
   for (int64_t K0 = 0; K0 < n; K0 += kOuterNB) {
-    const int set = (int)((K0 / kOuterNB) & 1);
-    // columns [c0, c1) right of the panel -= L21 U12
-    auto update = [&](int64_t kend, int64_t c0, int64_t c1) -> int {
-      if constexpr (sizeof(T) == 8)
-        if (i8 && n - kend >= kI8Rows) return i8_gemm_sub(c, set, at(K0, c0), at(kend, c0), lda, n - kend, c0 - kend, c1 - c0);
-      return gemm_sub<T>(c, at(kend, K0), at(K0, c0), at(kend, c0), lda, n - kend, c1 - c0, (int)(kend - K0));
-    };
     const int64_t kend = std::min<int64_t>(K0 + kOuterNB, n);
     const int64_t knext = std::min<int64_t>(kend + kOuterNB, n);   // next panel: columns [kend, knext)
     // (1) factor the panel's columns, full height
@@ -1249,15 +1210,14 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
     }
-    if constexpr (sizeof(T) == 8)
-      if (i8 && n - kend >= kI8Rows)
-        if (int rc = i8_slice_rows(c, set, at(kend, K0), lda, n - kend)) return rc;
     FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_panel, c->stream));
     // (2) the next panel's columns: P's swaps and U12 rows, then their update
     if (knext > kend) {
       FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream, c->ev_rest, 0));
       if (int rc = strip(K0, (int)(kend - K0), 0, 0, kend, knext)) return rc;
-      if (int rc = update(kend, kend, knext)) return rc;
+      if (int rc = gemm_sub_f32(c, at(kend, K0), at(K0, kend), at(kend, kend), lda, n - kend, knext - kend,
+                                    (int)(kend - K0)))
+        return rc;
     }
     // (3) on stream2: swaps left of P, U12 rows beyond the next panel, their update
     {
@@ -1265,7 +1225,9 @@ int lu_factor(fp_ctx* c, T* A, int64_t n, int64_t lda, int32_t* ipiv, float* cer
       FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream, c->ev_panel, 0));
       if (int rc = strip(K0, (int)(kend - K0), 0, K0, knext, n)) return rc;
       if (n > knext)
-        if (int rc = update(kend, knext, n)) return rc;
+        if (int rc = gemm_sub_f32(c, at(kend, K0), at(K0, knext), at(kend, knext), lda, n - kend, n - knext,
+                                      (int)(kend - K0)))
+            return rc;
       FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
     }
   }
@@ -2397,7 +2359,6 @@ int lu_solve_noalloc(fp_ctx* c, double* B, int64_t ldb, int64_t k) {
   return FP_OK;
 }
 
-template int lu_factor<double>(fp_ctx*, double*, int64_t, int64_t, int32_t*, float*);
 template int lu_factor<float>(fp_ctx*, float*, int64_t, int64_t, int32_t*, float*);
 template int lu_solve<double>(fp_ctx*, const double*, int64_t, int64_t, const int32_t*, double*, int64_t, int64_t, bool);
 template int lu_solve<float>(fp_ctx*, const float*, int64_t, int64_t, const int32_t*, float*, int64_t, int64_t, bool);
