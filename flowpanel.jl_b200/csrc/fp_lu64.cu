@@ -21,14 +21,14 @@ namespace p64 {
 
 constexpr int R = 64;                // rows of a CTA, columns of a block
 constexpr int W = kOuterPanel;       // columns of a panel
-constexpr int SUB = 16;              // columns factored by one warp at a time
+constexpr int SUB = 16;              // sub-blocks of the triangular solves
 // pitches of 4 (mod 16) doubles: the 4 x 4 elements that a half-warp of a DMMA
 // fragment reads fall in 16 different pairs of banks
 constexpr int PP = R + 4, VP = SUB + 4;
 constexpr int NT = 512;
 constexpr int VBLK = SUB * VP;       // one 16 x 16 inverse
 constexpr int SLOT = kLuNB * kLuNB;  // doubles of a block's slot: inverses of the four U, then of the four L sub-blocks
-constexpr size_t kSmem = (size_t)(W * PP + 2 * R * PP + 8 * VBLK + 2 * SUB) * 8 + 2 * R * 4 + 64;
+constexpr size_t kSmem = (size_t)(W * PP + 2 * R * PP + 8 * VBLK) * 8 + 2 * R * 4 + 16;
 constexpr int kSpin = 1 << 22;
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
@@ -44,19 +44,14 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void pair_bar(int warp) {   // the two warps 2 i, 2 i + 1
-  asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
-}
-
 struct Smem {
   double (*P)[PP];      // [panel column][row]
   double (*Q)[R][PP];   // two 64 x 64 operands, [column][row]
   double* VU;           // inverses of the block's 16 x 16 U sub-blocks, [q][column][k]
   double* VL;           // of its L sub-blocks, [q][k][row]
-  double* pv;           // the pivot row of a step, two copies
   int* pr;              // physical row of each logical row
   int* lp;              // logical position of each step's pivot
-  unsigned long long* used;   // rows taken as pivots after each sub-block, two copies
+  int* done;            // pivot steps made
   int* stop;
 };
 
@@ -71,167 +66,171 @@ __device__ __forceinline__ void load_block(double (*dst)[PP], const double* A, i
   }
 }
 
-// Columns J0 .. J0 + 15 of the diagonal block D ([column][row], 64 rows) by one
-// warp: lane l holds rows l and l + 32, their entries shifted so that a[0] is
-// the current column (a rolled loop: the code stays in the instruction cache).
-// The pivot is LAPACK's: the largest |a| among the rows not yet taken, the
-// first in logical order on ties. Each lane forms the reciprocals of its
-// own candidates while the search runs.
-__device__ __forceinline__ void factor_sub(Smem& s, double (*D)[PP], int J0, int nb, bool& used0, bool& used1, int& pos0,
-                                           int& pos1, bool& zero) {
-  const int lane = threadIdx.x & 31;
-  double a0[SUB], a1[SUB];
-#pragma unroll
-  for (int c = 0; c < SUB; ++c) {
-    a0[c] = D[J0 + c][lane];
-    a1[c] = D[J0 + c][lane + 32];
-  }
-#pragma unroll 1
-  for (int j = 0; j < SUB; ++j) {
-    const int J = J0 + j;
-    double* const pv = s.pv + (j & 1) * SUB;
-    const unsigned long long k0 = used0 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a0[0])) + 1ull;
-    const unsigned long long k1 = used1 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a1[0])) + 1ull;
-    const bool second = k1 > k0 || (k1 == k0 && pos1 < pos0);
-    const unsigned long long k = second ? k1 : k0;
-    const int pos = second ? pos1 : pos0;
-    const double r0 = a0[0] != 0.0 ? __drcp_rn(a0[0]) : 0.0, r1 = a1[0] != 0.0 ? __drcp_rn(a1[0]) : 0.0;
-    const unsigned hi = (unsigned)(k >> 32);
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned lo = hi == mh ? (unsigned)k : 0u;
-    const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-    const bool top = hi == mh && (unsigned)k == ml;
-    const unsigned lead = __reduce_min_sync(0xffffffffu, top ? (unsigned)((pos << 6) | (second ? 32 : 0) | lane) : ~0u);
-    const int src = lead & 31, lpos = (int)(lead >> 6);
-    const bool mine = lane == src, psec = (lead >> 5) & 1;
-    if (mine) {   // the pivot row to all lanes
-      double2* o = reinterpret_cast<double2*>(pv);
-#pragma unroll
-      for (int c = 0; c < SUB; c += 2) o[c / 2] = psec ? make_double2(a1[c], a1[c + 1]) : make_double2(a0[c], a0[c + 1]);
-    }
-    const double rp = __shfl_sync(0xffffffffu, psec ? r1 : r0, src);
-    const double p1 = __shfl_sync(0xffffffffu, psec ? a1[1] : a0[1], src);
-    zero |= J < nb && rp == 0.0;
-    // the pivot row takes logical place J, the row that had it the pivot's
-    if (mine && !psec) { used0 = true; pos0 = J; } else if (pos0 == J) { pos0 = lpos; }
-    if (mine && psec) { used1 = true; pos1 = J; } else if (pos1 == J) { pos1 = lpos; }
-    if (lane == 0) {
-      s.pr[J] = src + (psec ? 32 : 0);
-      s.lp[J] = lpos;
-    }
-    // multipliers; zero for rows already taken, which the updates below then leave alone
-    const double m0 = used0 ? 0.0 : a0[0] * rp, m1 = used1 ? 0.0 : a1[0] * rp;
-    a0[0] = fma(-m0, p1, a0[1]);   // the next column first: its search waits for it
-    a1[0] = fma(-m1, p1, a1[1]);
-    if (!used0) D[J][lane] = m0;
-    if (!used1) D[J][lane + 32] = m1;
-    __syncwarp();
-    double u[SUB];
-    const double2* in = reinterpret_cast<const double2*>(pv);
-#pragma unroll
-    for (int c = 0; c < SUB; c += 2) {
-      const double2 v = in[c / 2];
-      u[c] = v.x;
-      u[c + 1] = v.y;
-    }
-#pragma unroll
-    for (int c = 1; c < SUB - 1; ++c) {
-      a0[c] = fma(-m0, u[c + 1], a0[c + 1]);
-      a1[c] = fma(-m1, u[c + 1], a1[c + 1]);
-    }
-    if (lane < SUB - j) D[J + lane][src + (psec ? 32 : 0)] = pv[lane];   // the pivot's row of U
-  }
-  const unsigned b0 = __ballot_sync(0xffffffffu, used0), b1 = __ballot_sync(0xffffffffu, used1);
-  if (lane == 0) s.used[(J0 / SUB) & 1] = (unsigned long long)b1 << 32 | b0;
+// 1 / d for 2^-1000 <= |d| <= 2^1000: the hardware's approximation, a
+// third-order and a second-order Newton step. Straight-line code, so that a
+// warp's reciprocals overlap its pivot search.
+__device__ __forceinline__ double newton_rcp(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  double e = fma(-d, x, 1.0);
+  x = fma(x, fma(e, e, e), x);
+  e = fma(-d, x, 1.0);
+  return fma(x, e, x);
 }
 
-// inverse of the 16 x 16 unit lower (lane < 16) triangle of the logical rows
-// and columns J0.. of D, column i per lane, to VL[q][k = column][row]
-__device__ __forceinline__ void inv_lower(Smem& s, double (*D)[PP], int J0, int lane) {
-  if (lane >= SUB) return;
+// Inverses of the 16 x 16 triangles at logical rows and columns J0.. of D (row r
+// of it is row rowof(r) of D), column i per lane, by columns so that a step is
+// one FMA deep: the unit lower one to VL[q][k = column][row], the upper one to
+// VU[q][column][k].
+template <class RowOf>
+__device__ __forceinline__ void inv_lower(Smem& s, double (*D)[PP], int J0, int lane, RowOf rowof) {
   double x[SUB];
 #pragma unroll
-  for (int r = 0; r < SUB; ++r) {
-    double v = r == lane ? 1.0 : 0.0;
+  for (int r = 0; r < SUB; ++r) x[r] = r == lane ? 1.0 : 0.0;
 #pragma unroll
-    for (int k = 0; k < r; ++k) v = fma(-D[J0 + k][s.pr[J0 + r]], x[k], v);
-    x[r] = v;
+  for (int k = 0; k < SUB - 1; ++k)
+#pragma unroll
+    for (int r = k + 1; r < SUB; ++r) x[r] = fma(-D[J0 + k][rowof(J0 + r)], x[k], x[r]);
+  if (lane < SUB) {
+    double* o = s.VL + (J0 / SUB) * VBLK + lane * VP;
+#pragma unroll
+    for (int r = 0; r < SUB; ++r) o[r] = x[r];
   }
-  double* o = s.VL + (J0 / SUB) * VBLK + lane * VP;
-#pragma unroll
-  for (int r = 0; r < SUB; ++r) o[r] = x[r];
 }
-// inverse of the upper triangle, column i per lane, to VU[q][column][k]
-__device__ __forceinline__ void inv_upper(Smem& s, double (*D)[PP], int J0, int lane) {
-  if (lane >= SUB) return;
+template <class RowOf>
+__device__ __forceinline__ void inv_upper(Smem& s, double (*D)[PP], int J0, int lane, RowOf rowof) {
+  const double d = D[J0 + (lane & 15)][rowof(J0 + (lane & 15))];
+  const double rd = d != 0.0 ? __drcp_rn(d) : 0.0;
   double x[SUB];
 #pragma unroll
-  for (int r = SUB - 1; r >= 0; --r) {
-    double v = r == lane ? 1.0 : 0.0;
+  for (int r = 0; r < SUB; ++r) x[r] = r == lane ? 1.0 : 0.0;
 #pragma unroll
-    for (int k = SUB - 1; k > r; --k) v = fma(-D[J0 + k][s.pr[J0 + r]], x[k], v);
-    const double d = D[J0 + r][s.pr[J0 + r]];
-    x[r] = d != 0.0 ? v * __drcp_rn(d) : 0.0;
+  for (int k = SUB - 1; k >= 0; --k) {
+    x[k] *= __shfl_sync(0xffffffffu, rd, k);
+#pragma unroll
+    for (int r = 0; r < k; ++r) x[r] = fma(-D[J0 + k][rowof(J0 + r)], x[k], x[r]);
   }
-  double* o = s.VU + (J0 / SUB) * VBLK + lane * VP;
+  if (lane < SUB) {
+    double* o = s.VU + (J0 / SUB) * VBLK + lane * VP;
 #pragma unroll
-  for (int r = 0; r < SUB; ++r) o[r] = x[r];
+    for (int r = 0; r < SUB; ++r) o[r] = x[r];
+  }
 }
 
-// The CTA factors the 64 x 64 diagonal block D in place, rows never moving:
-// after each 16 columns the U rows of the columns right of them, then the
-// rank-16 update of the rows not yet taken, the next 16 columns first, so that
-// warp 0 goes on with them while the other warps finish. Last, D in logical
-// row order.
-__device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, int* status) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+// The CTA factors the 64 x 64 diagonal block D ([column][row]) in place, rows
+// never moving; last, D in logical row order, also to the matrix (Ad). Warp w
+// holds columns 4 w .. 4 w + 3 in registers, lane l of it rows l and l + 32. It
+// applies the pivots of the warps before it as they are published (the
+// multipliers are D's column itself, the pivot's entries of its own columns
+// come by shuffles), then makes its own four steps: so a step's chain, search
+// -> multipliers -> next column -> its search, stays inside one warp and carries no
+// other work. The pivot is LAPACK's: the largest |a| among the rows not yet
+// taken, the first in logical order on ties. One warp for 16 columns with the
+// products of the other columns between took 37 us a block.
+__device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, double* Ad, int64_t lda, int* status) {
+  constexpr int C = R / (NT / 32);   // columns of a warp
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, own = warp * C;
+  volatile int* const done = s.done;
+  double a0[C], a1[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    a0[c] = D[own + c][lane];
+    a1[c] = D[own + c][lane + 32];
+  }
   bool used0 = false, used1 = false, zero = false;
-  int pos0 = lane, pos1 = lane + 32;
-  // one 8 x 8 tile of the update of columns J1.. from the pivots J1 - 16 .. J1 - 1
-  auto tile = [&](int J1, int ct, int rt) {
-    const int row = rt * 8 + g, c0 = J1 + ct * 8;
-    double d0 = 0.0, d1 = 0.0;
-#pragma unroll
-    for (int k = 0; k < SUB; k += 4)
-      dmma(d0, d1, D[J1 - SUB + k + t][row], D[c0 + g][s.pr[J1 - SUB + k + t]]);
-    if (!((s.used[(J1 / SUB - 1) & 1] >> row) & 1)) {
-      D[c0 + 2 * t][row] -= d0;
-      D[c0 + 2 * t + 1][row] -= d1;
-    }
+  int pos0 = lane, pos1 = lane + 32, seen = 0;
+  auto wait_done = [&](int level) {
+    for (int i = 0; seen < level && i < kSpin; ++i) seen = *done;
+    __syncwarp();
+    asm volatile("" ::: "memory");
+  };
+  // the pivot row of step J takes logical place J, the row that had it the pivot's
+  auto take = [&](int J, int pr, int lpos) {
+    if (lane == pr) { used0 = true; pos0 = J; } else if (pos0 == J) { pos0 = lpos; }
+    if (lane + 32 == pr) { used1 = true; pos1 = J; } else if (pos1 == J) { pos1 = lpos; }
   };
 #pragma unroll 1
-  for (int q = 0; q < R / SUB; ++q) {
-    const int J0 = q * SUB, J1 = J0 + SUB, right = (R - J1) / 8;   // column tiles right of the sub-block
-    if (warp == 0) {
-      factor_sub(s, D, J0, nb, used0, used1, pos0, pos1, zero);
-    } else if (q > 0) {   // the columns beyond, of the previous step; the inverses of its sub-blocks
-      for (int i = 16 + warp - 1; i < R - J0; i += 15) tile(J0, i >> 3, i & 7);
-      if (warp == 14) inv_lower(s, D, J0 - SUB, lane);
-      if (warp == 15) inv_upper(s, D, J0 - SUB, lane);
+  for (int J = 0; J < own; ++J) {
+    wait_done(J + 1);
+    const int pr = s.pr[J], src = pr & 31;
+    const double l0 = D[J][lane], l1 = D[J][lane + 32];
+    take(J, pr, s.lp[J]);
+    const double m0 = used0 ? 0.0 : l0, m1 = used1 ? 0.0 : l1;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const double p = __shfl_sync(0xffffffffu, pr & 32 ? a1[c] : a0[c], src);
+      a0[c] = fma(-m0, p, a0[c]);
+      a1[c] = fma(-m1, p, a1[c]);
     }
-    __syncthreads();
-    if (right == 0) break;
-    if (tid < R - J1) {   // U rows of this sub-block: a column per thread
-      double* col = D[J1 + tid];
-      double u[SUB];
-#pragma unroll
-      for (int k = 0; k < SUB; ++k) u[k] = col[s.pr[J0 + k]];
-#pragma unroll
-      for (int k = 0; k < SUB - 1; ++k)
-#pragma unroll
-        for (int r = k + 1; r < SUB; ++r) u[r] = fma(-D[J0 + k][s.pr[J0 + r]], u[k], u[r]);
-#pragma unroll
-      for (int k = 1; k < SUB; ++k) col[s.pr[J0 + k]] = u[k];
-    }
-    __syncthreads();
-    tile(J1, warp >> 3, warp & 7);   // the next 16 columns
-    __syncthreads();
   }
-  if (warp == 0 && zero && lane == 0) atomicOr(status, (int)DEV_ZERO_PIVOT);
-  if (warp == 14) inv_lower(s, D, R - SUB, lane);
-  if (warp == 15) inv_upper(s, D, R - SUB, lane);
+#pragma unroll
+  for (int j = 0; j < C; ++j) {
+    const int J = own + j;
+    const unsigned long long k0 = used0 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a0[j])) + 1ull;
+    const unsigned long long k1 = used1 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a1[j])) + 1ull;
+    const bool second = k1 > k0 || (k1 == k0 && pos1 < pos0);   // the lane's better row
+    const unsigned hi = (unsigned)((second ? k1 : k0) >> 32), lo = (unsigned)(second ? k1 : k0);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const int pos = second ? pos1 : pos0;
+    double v[C];   // its entries from column J on
+#pragma unroll
+    for (int c = j; c < C; ++c) v[c] = second ? a1[c] : a0[c];
+    double rv = newton_rcp(v[j]);
+    const bool odd = !(fabs(v[j]) >= 0x1p-1000 && fabs(v[j]) <= 0x1p1000);
+    const unsigned sec = __ballot_sync(0xffffffffu, second), odds = __ballot_sync(0xffffffffu, odd);
+    unsigned win = __ballot_sync(0xffffffffu, hi == mh);
+    if ((win & (win - 1)) | (win & odds)) {   // several lanes share the high word, or newton_rcp does not reach
+      const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+      const bool top = hi == mh && lo == ml;
+      const unsigned first = __reduce_min_sync(0xffffffffu, top ? (unsigned)pos : ~0u);
+      win = __ballot_sync(0xffffffffu, top && (unsigned)pos == first);
+      if (odd) rv = v[j] != 0.0 ? __drcp_rn(v[j]) : 0.0;
+    }
+    const int src = __ffs(win) - 1;
+    const int pr = src + ((sec >> src) & 1) * 32;
+    const double rp = __shfl_sync(0xffffffffu, rv, src);
+    double p[C];
+#pragma unroll
+    for (int c = j + 1; c < C; ++c) p[c] = __shfl_sync(0xffffffffu, v[c], src);
+    const int lpos = __shfl_sync(0xffffffffu, pos, src);
+    take(J, pr, lpos);
+    zero |= J < nb && rp == 0.0;
+    // multipliers; zero for rows already taken, which the updates then leave alone
+    const double m0 = used0 ? 0.0 : a0[j] * rp, m1 = used1 ? 0.0 : a1[j] * rp;
+#pragma unroll
+    for (int c = j + 1; c < C; ++c) {
+      a0[c] = fma(-m0, p[c], a0[c]);
+      a1[c] = fma(-m1, p[c], a1[c]);
+    }
+    // column J is final: U in the rows taken, L in the others
+    D[J][lane] = used0 ? a0[j] : m0;
+    D[J][lane + 32] = used1 ? a1[j] : m1;
+    if (lane == 0) {
+      s.pr[J] = pr;
+      s.lp[J] = lpos;
+    }
+    __syncwarp();
+    __threadfence_block();
+    if (lane == 0) *done = J + 1;
+  }
+  if (zero && lane == 0) atomicOr(status, (int)DEV_ZERO_PIVOT);
+  // the inverses of the sub-blocks, as each is done
+  if (warp < 8) {
+    const int J0 = (warp >> 1) * SUB;
+    wait_done(J0 + SUB);
+    auto rowof = [&](int r) { return s.pr[r]; };
+    if (warp & 1) inv_upper(s, D, J0, lane, rowof);
+    else inv_lower(s, D, J0, lane, rowof);
+  }
+  __syncthreads();
   double (*L)[PP] = s.Q[0];
-  for (int e = tid; e < R * R; e += NT) L[e >> 6][e & 63] = D[e >> 6][s.pr[e & 63]];
+  for (int e = tid; e < R * R; e += NT) {
+    const int col = e >> 6, r = e & 63;
+    const double x = D[col][s.pr[r]];
+    L[col][r] = x;
+    if (r < nb && col < nb) Ad[col * lda + r] = x;
+  }
+  if (tid == 0) *done = 0;
   __syncthreads();
   for (int e = tid; e < R * R; e += NT) D[e >> 6][e & 63] = L[e >> 6][e & 63];
 }
@@ -260,67 +259,89 @@ __device__ __forceinline__ void update(double (*C)[PP], double (*X)[PP], double 
 }
 
 // X (64 columns of the panel, [column][row]) <- X U^-1 by 16-column sub-blocks:
-// U in Q ([column][k]), the inverses of its diagonal sub-blocks in VU. Two
-// warps an 8-row tile, 8 columns of a sub-block each. Returns max|X|.
+// U in Q ([column][k]), the inverses of its diagonal sub-blocks in VU. Eight
+// warps, an 8-row tile each, which depends on no other (no barriers). Returns
+// max|X|.
 __device__ __forceinline__ double solve_l21(double (*X)[PP], double (*Q)[PP], const double* VU) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int row = (warp >> 1) * 8 + g, half = (warp & 1) * 8;
+  if (warp >= 8) return 0.0;
+  const int row = warp * 8 + g;
   double mx = 0.0;
 #pragma unroll 1
   for (int q = 0; q < R / SUB; ++q) {
-    const int c = q * SUB + half;
-    double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
+    const int c = q * SUB;
+    double d[2][2][2] = {};   // [half][chain]
 #pragma unroll 2
-    for (int k = 0; k < q * SUB; k += 8) {
-      dmma(d0, d1, X[k + t][row], Q[c + g][k + t]);
-      dmma(e0, e1, X[k + 4 + t][row], Q[c + g][k + 4 + t]);
+    for (int k = 0; k < c; k += 8)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const double a = X[k + 4 * i + t][row];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) dmma(d[h][i][0], d[h][i][1], a, Q[c + 8 * h + g][k + 4 * i + t]);
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) X[c + 8 * h + 2 * t + e][row] -= d[h][0][e] + d[h][1][e];
+    __syncwarp();
+    double z[2][2][2] = {};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double a = X[c + 4 * k + t][row];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) dmma(z[h][k & 1][0], z[h][k & 1][1], a, VU[q * VBLK + (8 * h + g) * VP + 4 * k + t]);
     }
-    X[c + 2 * t][row] -= d0 + e0;
-    X[c + 2 * t + 1][row] -= d1 + e1;
-    pair_bar(warp);
-    double a[4];
+    __syncwarp();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] = X[q * SUB + 4 * k + t][row];
-    d0 = d1 = 0.0;
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) dmma(d0, d1, a[k], VU[q * VBLK + (half + g) * VP + 4 * k + t]);
-    pair_bar(warp);
-    X[c + 2 * t][row] = d0;
-    X[c + 2 * t + 1][row] = d1;
-    mx = fmax(mx, fmax(fabs(d0), fabs(d1)));
-    pair_bar(warp);
+      for (int e = 0; e < 2; ++e) {
+        const double v = z[h][0][e] + z[h][1][e];
+        X[c + 8 * h + 2 * t + e][row] = v;
+        mx = fmax(mx, fabs(v));
+      }
+    __syncwarp();
   }
   return mx;
 }
 
-// Y (64 columns, [column][row], logical rows) <- L^-1 Y by 16-row sub-blocks: L in
-// the panel's columns ([k][row]), the inverses of its sub-blocks in VL. Two
-// warps an 8-column tile, 8 rows of a sub-block each.
-__device__ __forceinline__ void solve_u12(double (*Y)[PP], double (*L)[PP], const double* VL) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int c = (warp >> 1) * 8, half = (warp & 1) * 8;
+// Y (columns [column][row], logical rows) <- L^-1 Y by 16-row sub-blocks, the 8
+// columns y0.. of one warp: L [k][row], the inverses of its sub-blocks in VL
+template <int YP>
+__device__ __forceinline__ void solve_u12(double (*Y)[YP], int y0, int row0, double (*L)[PP], const double* VL) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const double* y = Y[y0 + g] + row0;
+  double* o[2] = {Y[y0 + 2 * t] + row0, Y[y0 + 2 * t + 1] + row0};
 #pragma unroll 1
   for (int q = 0; q < R / SUB; ++q) {
-    const int r = q * SUB + half + g;
-    double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
+    const int r = q * SUB;
+    double d[2][2][2] = {};
 #pragma unroll 2
-    for (int k = 0; k < q * SUB; k += 8) {
-      dmma(d0, d1, L[k + t][r], Y[c + g][k + t]);
-      dmma(e0, e1, L[k + 4 + t][r], Y[c + g][k + 4 + t]);
+    for (int k = 0; k < r; k += 8)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const double b = y[k + 4 * i + t];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) dmma(d[h][i][0], d[h][i][1], L[k + 4 * i + t][r + 8 * h + g], b);
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) o[e][r + 8 * h + g] -= d[h][0][e] + d[h][1][e];
+    __syncwarp();
+    double z[2][2][2] = {};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const double b = y[r + 4 * k + t];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) dmma(z[h][k & 1][0], z[h][k & 1][1], VL[q * VBLK + (4 * k + t) * VP + 8 * h + g], b);
     }
-    Y[c + 2 * t][r] -= d0 + e0;
-    Y[c + 2 * t + 1][r] -= d1 + e1;
-    pair_bar(warp);
-    double b[4];
+    __syncwarp();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) b[k] = Y[c + g][q * SUB + 4 * k + t];
-    d0 = d1 = 0.0;
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) dmma(d0, d1, VL[q * VBLK + (4 * k + t) * VP + half + g], b[k]);
-    pair_bar(warp);
-    Y[c + 2 * t][r] = d0;
-    Y[c + 2 * t + 1][r] = d1;
-    pair_bar(warp);
+      for (int e = 0; e < 2; ++e) o[e][r + 8 * h + g] = z[h][0][e] + z[h][1][e];
+    __syncwarp();
   }
 }
 
@@ -343,15 +364,15 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
   s.Q = reinterpret_cast<double (*)[R][PP]>(p); p += 2 * R * PP;
   s.VU = p; p += 4 * VBLK;
   s.VL = p; p += 4 * VBLK;
-  s.pv = p; p += 2 * SUB;
-  s.used = reinterpret_cast<unsigned long long*>(p); p += 2;
-  s.stop = reinterpret_cast<int*>(p); p += 1;
   s.pr = reinterpret_cast<int*>(p);
   s.lp = s.pr + R;
+  s.done = s.lp + R;
+  s.stop = s.done + 1;
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid == 0) {
     s.lp[0] = (int)(atomicAdd(sync, 1u) - ticket0);
     *s.stop = 0;
+    *s.done = 0;
   }
   __syncthreads();
   const int c = s.lp[0];
@@ -388,7 +409,7 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
       flags[c] = flag0 + level;
     }
   };
-  // factor this CTA's diagonal block, write it and the rows left of it, publish
+  // factor this CTA's diagonal block and publish it
   auto diagonal = [&]() {
     double (*D)[PP] = s.P + c * R;
     const int nb = rows;
@@ -397,12 +418,8 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
         if ((e & 63) >= nb) D[e >> 6][e & 63] = (e >> 6) == (e & 63) ? 1.0 : 0.0;
       __syncthreads();
     }
-    factor_diag(s, D, nb, status);
+    factor_diag(s, D, nb, A + r0 * lda + r0, lda, status);
     __syncthreads();
-    for (int e = tid; e < R * R; e += NT) {
-      const int col = e >> 6, r = e & 63;
-      if (r < nb && col < nb) A[(r0 + col) * lda + r0 + r] = D[col][r];
-    }
     double* slot = slots + (size_t)c * SLOT;
     for (int e = tid; e < 4 * SUB * SUB; e += NT) {
       const int q = e >> 8, i = (e >> 4) & 15, k = e & 15;
@@ -410,13 +427,16 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
       slot[4 * SUB * SUB + e] = s.VL[q * VBLK + i * VP + k];
     }
     publish(1);
+  };
+  // what no other CTA waits for: the pivots, and the rows left of the block in their order
+  auto rest = [&]() {
     if (tid < R) {
       rowat[c * R + tid] = s.pr[tid];
-      if (tid < nb) ipiv[r0 + tid] = (int32_t)(r0 + s.lp[tid]);
+      if (tid < rows) ipiv[r0 + tid] = (int32_t)(r0 + s.lp[tid]);
     }
     for (int e = tid; e < c * R * R; e += NT) {
       const int col = e >> 6, r = e & 63;
-      if (r < nb) A[(K0 + col) * lda + r0 + r] = s.P[col][s.pr[r]];
+      if (r < rows) A[(K0 + col) * lda + r0 + r] = s.P[col][s.pr[r]];
     }
   };
   // this CTA's rows of U in column block j, from its updated rows
@@ -424,7 +444,7 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
     __syncthreads();
     for (int e = tid; e < R * R; e += NT) Y[e >> 6][e & 63] = s.P[j * R + (e >> 6)][s.pr[e & 63]];
     __syncthreads();
-    solve_u12(Y, s.P + c * R, s.VL);
+    if (tid < 256) solve_u12<PP>(Y, (tid >> 5) * 8, 0, s.P + c * R, s.VL);
     __syncthreads();
     for (int e = tid; e < R * R; e += NT) {
       const int col = e >> 6, r = e & 63;
@@ -437,6 +457,7 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
     diagonal();
     cp_wait<0>();
     for (int j = 1; j < nblk; ++j) u12(j, s.Q[j & 1]);
+    rest();
     return;
   }
   const int steps = min(c, nblk);
@@ -471,7 +492,9 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
     if (!ok) break;
     __syncthreads();
   }
-  if (c >= nblk)   // rows below the panel's blocks: L21
+  if (c < nblk)
+    rest();
+  else   // rows below the panel's blocks: L21
     for (int e = tid; e < nblk * R * R; e += NT) {
       const int col = e >> 6, r = e & 63;
       if (r < rows && col < w) A[(K0 + col) * lda + r0 + r] = s.P[col][r];
@@ -543,36 +566,8 @@ k_strip64(double* __restrict__ A, int64_t lda, int64_t K0, int w, const double* 
       if (nb < nblk) { stage((i + 1) & 1, nb2, nb); cp_wait<1>(); } else { cp_wait<0>(); }
       __syncthreads();
       double (*Lb)[PP] = L[i & 1];
-      if (b2 == b) {   // U_b: warps 0..3, an 8-column tile each pair, 8 rows of a sub-block each
-        if (warp < 4) {
-          const int c = (warp >> 1) * 8, half = (warp & 1) * 8;
-#pragma unroll 1
-          for (int q = 0; q < R / SUB; ++q) {
-            const int r = q * SUB + half + g;
-            double* x0 = X[c + 2 * t] + b * R + r;
-            double* x1 = X[c + 2 * t + 1] + b * R + r;
-            const double* y = X[c + g] + b * R;
-            double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll 2
-            for (int k = 0; k < q * SUB; k += 8) {
-              dmma(d0, d1, Lb[k + t][r], y[k + t]);
-              dmma(e0, e1, Lb[k + 4 + t][r], y[k + 4 + t]);
-            }
-            *x0 -= d0 + e0;
-            *x1 -= d1 + e1;
-            pair_bar(warp);
-            double v[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v[k] = y[q * SUB + 4 * k + t];
-            d0 = d1 = 0.0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) dmma(d0, d1, V[q * VBLK + (4 * k + t) * VP + half + g], v[k]);
-            pair_bar(warp);
-            *x0 = d0;
-            *x1 = d1;
-            pair_bar(warp);
-          }
-        }
+      if (b2 == b) {   // U_b, an 8-column tile a warp
+        if (warp < COLS / 8) solve_u12<XP>(X, warp * 8, b * R, Lb, V);
       } else {   // X_b2 -= L(b2, b) U_b: a row tile a warp, both column tiles
         const int r = warp * 8 + g;
         double d[2][2] = {};
