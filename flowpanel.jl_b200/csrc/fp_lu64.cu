@@ -28,7 +28,7 @@ constexpr int PP = R + 4, VP = SUB + 4;
 constexpr int NT = 512;
 constexpr int VBLK = SUB * VP;       // one 16 x 16 inverse
 constexpr int SLOT = kLuNB * kLuNB;  // doubles of a block's slot: inverses of the four U, then of the four L sub-blocks
-constexpr size_t kSmem = (size_t)(W * PP + 2 * R * PP + 8 * VBLK) * 8 + 2 * R * 4 + 16;
+constexpr size_t kSmem = (size_t)(W * PP + 2 * R * PP + 8 * VBLK + R) * 8 + 2 * R * 4 + 16;
 constexpr int kSpin = 1 << 22;
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
@@ -44,6 +44,23 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// waits (bounded) for a pivot step's barrier
+__device__ __forceinline__ void wait_step(uint64_t* bar) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
+  for (int i = 0; i < (1 << 16); ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(a)
+        : "memory");
+    if (ok) break;
+  }
+  __syncwarp();
+}
+
 struct Smem {
   double (*P)[PP];      // [panel column][row]
   double (*Q)[R][PP];   // two 64 x 64 operands, [column][row]
@@ -51,7 +68,7 @@ struct Smem {
   double* VL;           // of its L sub-blocks, [q][k][row]
   int* pr;              // physical row of each logical row
   int* lp;              // logical position of each step's pivot
-  int* done;            // pivot steps made
+  uint64_t* step;       // one barrier a pivot step: its column and pivot row are written
   int* stop;
 };
 
@@ -130,7 +147,6 @@ __device__ __forceinline__ void inv_upper(Smem& s, double (*D)[PP], int J0, int 
 __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, double* Ad, int64_t lda, int* status) {
   constexpr int C = R / (NT / 32);   // columns of a warp
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, own = warp * C;
-  volatile int* const done = s.done;
   double a0[C], a1[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) {
@@ -138,12 +154,7 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
     a1[c] = D[own + c][lane + 32];
   }
   bool used0 = false, used1 = false, zero = false;
-  int pos0 = lane, pos1 = lane + 32, seen = 0;
-  auto wait_done = [&](int level) {
-    for (int i = 0; seen < level && i < kSpin; ++i) seen = *done;
-    __syncwarp();
-    asm volatile("" ::: "memory");
-  };
+  int pos0 = lane, pos1 = lane + 32;
   // the pivot row of step J takes logical place J, the row that had it the pivot's
   auto take = [&](int J, int pr, int lpos) {
     if (lane == pr) { used0 = true; pos0 = J; } else if (pos0 == J) { pos0 = lpos; }
@@ -151,7 +162,7 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
   };
 #pragma unroll 1
   for (int J = 0; J < own; ++J) {
-    wait_done(J + 1);
+    wait_step(s.step + J);
     const int pr = s.pr[J], src = pr & 31;
     const double l0 = D[J][lane], l1 = D[J][lane + 32];
     take(J, pr, s.lp[J]);
@@ -163,19 +174,28 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
       a1[c] = fma(-m1, p, a1[c]);
     }
   }
+  // the search in column own + j: the lane's better row, the warp's largest high
+  // word, the reciprocal of the lane's candidate
+  bool second;
+  unsigned hi, lo, mh;
+  double rv;
+  auto search = [&](double x0, double x1) {
+    const unsigned long long k0 = used0 ? 0ull : (unsigned long long)__double_as_longlong(fabs(x0)) + 1ull;
+    const unsigned long long k1 = used1 ? 0ull : (unsigned long long)__double_as_longlong(fabs(x1)) + 1ull;
+    second = k1 > k0 || (k1 == k0 && pos1 < pos0);
+    hi = (unsigned)((second ? k1 : k0) >> 32);
+    lo = (unsigned)(second ? k1 : k0);
+    mh = __reduce_max_sync(0xffffffffu, hi);
+    rv = newton_rcp(second ? x1 : x0);
+  };
+  search(a0[0], a1[0]);
 #pragma unroll
   for (int j = 0; j < C; ++j) {
     const int J = own + j;
-    const unsigned long long k0 = used0 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a0[j])) + 1ull;
-    const unsigned long long k1 = used1 ? 0ull : (unsigned long long)__double_as_longlong(fabs(a1[j])) + 1ull;
-    const bool second = k1 > k0 || (k1 == k0 && pos1 < pos0);   // the lane's better row
-    const unsigned hi = (unsigned)((second ? k1 : k0) >> 32), lo = (unsigned)(second ? k1 : k0);
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
     const int pos = second ? pos1 : pos0;
-    double v[C];   // its entries from column J on
+    double v[C];   // the lane's candidate's entries from column J on
 #pragma unroll
     for (int c = j; c < C; ++c) v[c] = second ? a1[c] : a0[c];
-    double rv = newton_rcp(v[j]);
     const bool odd = !(fabs(v[j]) >= 0x1p-1000 && fabs(v[j]) <= 0x1p1000);
     const unsigned sec = __ballot_sync(0xffffffffu, second), odds = __ballot_sync(0xffffffffu, odd);
     unsigned win = __ballot_sync(0xffffffffu, hi == mh);
@@ -203,21 +223,24 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
       a1[c] = fma(-m1, p[c], a1[c]);
     }
     // column J is final: U in the rows taken, L in the others
-    D[J][lane] = used0 ? a0[j] : m0;
-    D[J][lane + 32] = used1 ? a1[j] : m1;
+    const double f0 = used0 ? a0[j] : m0, f1 = used1 ? a1[j] : m1;
+    if (j + 1 < C) search(a0[j + 1 < C ? j + 1 : 0], a1[j + 1 < C ? j + 1 : 0]);   // before the stores: the chain waits for it
+    D[J][lane] = f0;
+    D[J][lane + 32] = f1;
     if (lane == 0) {
       s.pr[J] = pr;
       s.lp[J] = lpos;
     }
     __syncwarp();
-    __threadfence_block();
-    if (lane == 0) *done = J + 1;
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(s.step + J))
+                   : "memory");
   }
   if (zero && lane == 0) atomicOr(status, (int)DEV_ZERO_PIVOT);
   // the inverses of the sub-blocks, as each is done
   if (warp < 8) {
     const int J0 = (warp >> 1) * SUB;
-    wait_done(J0 + SUB);
+    wait_step(s.step + J0 + SUB - 1);
     auto rowof = [&](int r) { return s.pr[r]; };
     if (warp & 1) inv_upper(s, D, J0, lane, rowof);
     else inv_lower(s, D, J0, lane, rowof);
@@ -230,7 +253,6 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
     L[col][r] = x;
     if (r < nb && col < nb) Ad[col * lda + r] = x;
   }
-  if (tid == 0) *done = 0;
   __syncthreads();
   for (int e = tid; e < R * R; e += NT) D[e >> 6][e & 63] = L[e >> 6][e & 63];
 }
@@ -364,15 +386,16 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
   s.Q = reinterpret_cast<double (*)[R][PP]>(p); p += 2 * R * PP;
   s.VU = p; p += 4 * VBLK;
   s.VL = p; p += 4 * VBLK;
+  s.step = reinterpret_cast<uint64_t*>(p); p += R;
   s.pr = reinterpret_cast<int*>(p);
   s.lp = s.pr + R;
-  s.done = s.lp + R;
-  s.stop = s.done + 1;
+  s.stop = s.lp + R;
   const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < R)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(s.step + tid)) : "memory");
   if (tid == 0) {
     s.lp[0] = (int)(atomicAdd(sync, 1u) - ticket0);
     *s.stop = 0;
-    *s.done = 0;
   }
   __syncthreads();
   const int c = s.lp[0];
