@@ -161,27 +161,44 @@ def _panel_arrays(mesh: Mesh):
     offs = mesh.panel_offsets
     nn = np.diff(offs)
     idx = np.zeros((mesh.npanels, 4), np.int64)
+    if nn.size and (nn == nn[0]).all():
+        idx[:, :nn[0]] = np.reshape(mesh.panel_nodes[offs[0]:offs[-1]], (-1, nn[0]))
+        return idx, nn
     for k in range(4):
         sel = nn > k
         idx[sel, k] = mesh.panel_nodes[offs[:-1][sel] + k]
     return idx, nn
 
 
+# The geometry works on coordinate arrays (x, y, z of one kind each), a third of
+# the time of the same operations on (N, 3) rows.
+def _cross(a, b):
+    return a[1] * b[2] - a[2] * b[1], a[2] * b[0] - a[0] * b[2], a[0] * b[1] - a[1] * b[0]
+
+
+def _unit(a):
+    norm = np.sqrt(a[0] * a[0] + a[1] * a[1] + a[2] * a[2])
+    return tuple(x / norm for x in a)
+
+
 def _frame(mesh: Mesh):
+    """Coordinates of the nodes [coordinate][local node], t, o, n of every panel
+    (a tuple of coordinates each), node counts."""
     idx, nn = _panel_arrays(mesh)
-    P = mesh.nodes
-    e = P[idx[:, 1]] - P[idx[:, 0]]
-    f = P[idx[:, 2]] - P[idx[:, 0]]
-    t = e / np.linalg.norm(e, axis=1)[:, None]
-    c = np.cross(e, f)
-    n = c / np.linalg.norm(c, axis=1)[:, None]
-    o = np.cross(n, t)
-    return t, o, n, idx, nn
+    idx = np.ascontiguousarray(idx.T)
+    P = [np.take(np.ascontiguousarray(mesh.nodes[:, d]), idx) for d in range(3)]
+    t = _unit([p[1] - p[0] for p in P])
+    n = _unit(_cross([p[1] - p[0] for p in P], [p[2] - p[0] for p in P]))
+    return P, t, _cross(n, t), n, nn
 
 
 def calc_normals(body: AbstractBody, flipbyCPoffset=False):
     """Unit normals (N, 3) (src/FLOWPanel_abstractbody.jl:738-776)."""
-    _, _, n, _, _ = _frame(body.mesh)
+    return _normals(body, _frame(body.mesh), flipbyCPoffset)
+
+
+def _normals(body, frame, flipbyCPoffset=False):
+    n = np.stack(frame[3], axis=1)
     if flipbyCPoffset:
         if isinstance(body, MultiBody):
             s = body._cp_off_vector(1.0)
@@ -191,26 +208,36 @@ def calc_normals(body: AbstractBody, flipbyCPoffset=False):
     return n
 
 
+def _cp_offset(body: AbstractBody):
+    """off * l of every panel's control point, for the body's own offset."""
+    offv = body._default_off() if isinstance(body, MultiBody) else np.full(body.ncells, body.CPoffset)
+    return offv * body._l_vector(body.characteristiclength if not isinstance(body, MultiBody) else None)
+
+
 def calc_controlpoints(body: AbstractBody, normals=None, off=None, characteristiclength=None):
     """Control points (N, 3): vertex mean, in-plane centroid correction, then
     + off * l * n (src/FLOWPanel_abstractbody.jl:635-694)."""
-    t, o, n, idx, nn = _frame(body.mesh)
-    normals = n if normals is None else normals
-    P = body.mesh.nodes
-    mask = (np.arange(4)[None, :] < nn[:, None]).astype(float)
-    pts = P[idx] * mask[:, :, None]
-    c = pts.sum(axis=1) / nn[:, None]
-    d = (P[idx] - c[:, None, :]) * mask[:, :, None]
-    x = np.einsum("pkd,pd->p", d, t) / nn
-    y = np.einsum("pkd,pd->p", d, o) / nn
-    c = c + x[:, None] * t + y[:, None] * o
+    return _controlpoints(body, _frame(body.mesh), normals, off, characteristiclength)
+
+
+def _controlpoints(body, frame, normals=None, off=None, characteristiclength=None):
+    P, t, o, n, nn = frame
+    normals = np.stack(n, axis=1) if normals is None else normals
+    quad = nn > 3
+    corners = 4 if quad.any() else 3
+    c = [(p[0] + p[1] + p[2] + (np.where(quad, p[3], 0.0) if corners == 4 else 0.0)) / nn for p in P]
+    x = y = 0.0
+    for k in range(corners):
+        d = [p[k] - m for p, m in zip(P, c)]
+        u, v = (d[0] * e[0] + d[1] * e[1] + d[2] * e[2] for e in (t, o))
+        x, y = (x + u, y + v) if k < 3 else (x + quad * u, y + quad * v)
+    x, y = x / nn, y / nn
+    c = np.stack([m + x * a + y * b for m, a, b in zip(c, t, o)], axis=1)
     if off is None:
-        offv = body._default_off() if isinstance(body, MultiBody) else np.full(body.ncells, body.CPoffset)
-        l = body._l_vector(body.characteristiclength if not isinstance(body, MultiBody) else None)
+        offl = _cp_offset(body)
     else:
-        offv = body._cp_off_vector(off)
-        l = body._l_vector(characteristiclength)
-    return c + (offv * l)[:, None] * normals
+        offl = body._cp_off_vector(off) * body._l_vector(characteristiclength)
+    return c + offl[:, None] * normals
 
 
 def calc_areas(body: AbstractBody):
@@ -255,12 +282,11 @@ class B200Solver:
         self.tuned = {}   # (N, precision) -> knob values chosen by fp_autotune
 
     def load(self, body: AbstractBody, normals=None, CPs=None):
+        """Normals and control points that are not given are formed on the device
+        (those of calc_normals and calc_controlpoints)."""
         m = body.mesh
-        if normals is None:
-            normals = calc_normals(body)
-        if CPs is None:
-            CPs = calc_controlpoints(body, normals)
-        self.ctx.set_geometry(m.nodes, m.panel_offsets, m.panel_nodes, CPs, normals)
+        off = _cp_offset(body) if CPs is None else None
+        self.ctx.set_geometry(m.nodes, m.panel_offsets, m.panel_nodes, CPs, normals, off)
         self._geom_of = id(body)
 
     def close(self):
@@ -422,9 +448,8 @@ def calcfield_U(sourcebody: AbstractBody, targetbody: AbstractBody, offset=None,
     if not targetbody.check_field("Uinf"):
         raise RuntimeError("Target body doesn't have freestream field `\"Uinf\"`.")
     Uinfs = np.asarray(targetbody.get_field("Uinf")["field_data"], float)
-    normals = calc_normals(targetbody)
-    cps = calc_controlpoints(targetbody, normals, off=offset, characteristiclength=characteristiclength) \
-        if offset is not None else calc_controlpoints(targetbody, normals)
+    cps = _controlpoints(targetbody, _frame(targetbody.mesh), None, offset,
+                         characteristiclength if offset is not None else None)
     out = np.array(Uinfs, dtype=np.float64, copy=True)
     out = Uind(sourcebody, cps, out, solver)
     if addfield:

@@ -60,22 +60,6 @@ int consume_status(fp_ctx* c) {
 }
 
 // Panel unit vectors of docs/src/elements/paneldefinition.md:15-35.
-void frame(const double* nodes, const int32_t* pn, double t[3], double o[3], double n[3]) {
-  const double* a = nodes + 3 * (int64_t)pn[0];
-  const double* b = nodes + 3 * (int64_t)pn[1];
-  const double* c = nodes + 3 * (int64_t)pn[2];
-  double e[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
-  double f[3] = {c[0] - a[0], c[1] - a[1], c[2] - a[2]};
-  double ne = std::sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-  for (int k = 0; k < 3; ++k) t[k] = e[k] / ne;
-  double cr[3] = {e[1] * f[2] - e[2] * f[1], e[2] * f[0] - e[0] * f[2], e[0] * f[1] - e[1] * f[0]};
-  double nc = std::sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-  for (int k = 0; k < 3; ++k) n[k] = cr[k] / nc;
-  o[0] = n[1] * t[2] - n[2] * t[1];
-  o[1] = n[2] * t[0] - n[0] * t[2];
-  o[2] = n[0] * t[1] - n[1] * t[0];
-}
-
 int ensure_rhs(fp_ctx* c, int64_t k) {
   if (k <= c->cap_rhs) return FP_OK;
   dfree(c->d_rhs); dfree(c->d_x); dfree(c->d_r); dfree(c->d_w32); dfree(c->d_norms);
@@ -197,6 +181,7 @@ int fp_ctx_destroy(fp_ctx* c) {
   free_matrices(c);
   post_free(c);
   dfree(c->d_panels); dfree(c->d_src); dfree(c->d_tgt); dfree(c->d_wake);
+  dfree(c->d_geo);
   dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket); dfree(c->d_p64);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -264,65 +249,6 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
   c->assembled = -1;
   c->factored = -1;
 
-  std::vector<PanelRec> pr(npanels);
-  std::vector<SourceRec> sr(npanels);
-  std::vector<double> tgt(6 * npanels);
-  for (int64_t p = 0; p < npanels; ++p) {
-    const int32_t* pn = pnodes + offsets[p];
-    const int nn = offsets[p + 1] - offsets[p];
-    PanelRec& r = pr[p];
-    std::memset(&r, 0, sizeof(r));
-    for (int k = 0; k < nn; ++k)
-      for (int d = 0; d < 3; ++d) r.p[3 * k + d] = nodes[3 * (int64_t)pn[k] + d];
-    r.nn = nn;
-    double t[3], o[3], n[3];
-    frame(nodes, pn, t, o, n);
-    // source record: flipped frame (o, t, -n) of src/FLOWPanel_elements.jl:51-56
-    SourceRec& s = sr[p];
-    std::memset(&s, 0, sizeof(s));
-    s.nn = nn;
-    const double* O = nodes + 3 * (int64_t)pn[0];
-    for (int d = 0; d < 3; ++d) { s.O[d] = O[d]; s.t[d] = o[d]; s.o[d] = t[d]; s.n[d] = -n[d]; }
-    for (int k = 0; k < nn; ++k) {
-      const double* P = nodes + 3 * (int64_t)pn[k];
-      s.xs[k] = s.t[0] * (P[0] - O[0]) + s.t[1] * (P[1] - O[1]) + s.t[2] * (P[2] - O[2]);
-      s.ys[k] = s.o[0] * (P[0] - O[0]) + s.o[1] * (P[1] - O[1]) + s.o[2] * (P[2] - O[2]);
-      s.zs[k] = s.n[0] * (P[0] - O[0]) + s.n[1] * (P[1] - O[1]) + s.n[2] * (P[2] - O[2]);
-    }
-    for (int k = 0; k < nn; ++k) {
-      const int j = (k + 1) % nn;
-      const double dx = s.xs[j] - s.xs[k], dy = s.ys[j] - s.ys[k], dz = s.zs[j] - s.zs[k];
-      s.dij[k] = std::sqrt(dx * dx + dy * dy + dz * dz);
-      s.S[k] = (s.ys[j] - s.ys[k]) / s.dij[k];
-      s.Cc[k] = (s.xs[j] - s.xs[k]) / s.dij[k];
-    }
-    // control point and normal
-    double cp[3], nr[3];
-    if (normals) { for (int d = 0; d < 3; ++d) nr[d] = normals[3 * p + d]; }
-    else { for (int d = 0; d < 3; ++d) nr[d] = n[d]; }
-    if (cps) {
-      for (int d = 0; d < 3; ++d) cp[d] = cps[3 * p + d];
-    } else {
-      // _calc_controlpoints!: vertex mean, in-plane centroid correction, + off*l*n (l = 1)
-      double cc[3] = {0, 0, 0};
-      for (int k = 0; k < nn; ++k)
-        for (int d = 0; d < 3; ++d) cc[d] += nodes[3 * (int64_t)pn[k] + d];
-      for (int d = 0; d < 3; ++d) cc[d] /= nn;
-      double x = 0, y = 0;
-      for (int k = 0; k < nn; ++k) {
-        const double* P = nodes + 3 * (int64_t)pn[k];
-        for (int d = 0; d < 3; ++d) x += (P[d] - cc[d]) * t[d];
-        for (int d = 0; d < 3; ++d) y += (P[d] - cc[d]) * o[d];
-      }
-      x /= nn; y /= nn;
-      const double off = cp_offset ? cp_offset[p] : 1e-14;
-      for (int d = 0; d < 3; ++d) cp[d] = cc[d] + x * t[d] + y * o[d] + off * 1.0 * nr[d];
-    }
-    for (int d = 0; d < 3; ++d) {
-      tgt[d * npanels + p] = cp[d];
-      tgt[(3 + d) * npanels + p] = nr[d];
-    }
-  }
   if (npanels > c->cap_geom) {
     dfree(c->d_panels); dfree(c->d_src); dfree(c->d_tgt);
     c->cap_geom = 0;
@@ -331,11 +257,38 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
     FP_CUDA_TRY(c->err, cudaMalloc(&c->d_tgt, 6 * npanels * sizeof(double)));
     c->cap_geom = npanels;
   }
-  FP_CUDA_TRY(c->err, cudaMemcpyAsync(c->d_panels, pr.data(), npanels * sizeof(PanelRec), cudaMemcpyHostToDevice, c->stream));
-  FP_CUDA_TRY(c->err, cudaMemcpyAsync(c->d_src, sr.data(), npanels * sizeof(SourceRec), cudaMemcpyHostToDevice, c->stream));
-  FP_CUDA_TRY(c->err, cudaMemcpyAsync(c->d_tgt, tgt.data(), 6 * npanels * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  c->h_tgt = tgt;
-  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));
+  // the caller's arrays to one device buffer, the panel records from there (k_geometry)
+  const size_t nidx = (size_t)npanels + 1 + offsets[npanels];
+  const size_t words = 3 * (size_t)nnodes + (cps ? 3 * (size_t)npanels : 0) + (normals ? 3 * (size_t)npanels : 0) +
+                       (cp_offset ? (size_t)npanels : 0) + (nidx + 1) / 2;
+  if (words > c->cap_geo) {
+    dfree(c->d_geo);
+    c->cap_geo = 0;
+    FP_CUDA_TRY(c->err, cudaMalloc(&c->d_geo, words * sizeof(double)));
+    c->cap_geo = words;
+  }
+  double* at = c->d_geo;
+  auto put = [&](const double* src, size_t n) -> const double* {
+    if (!src) return nullptr;
+    double* dst = at;
+    at += n;
+    return cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyHostToDevice, c->stream) == cudaSuccess ? dst : nullptr;
+  };
+  GeometryArgs g;
+  g.nodes = put(nodes, 3 * (size_t)nnodes);
+  g.cps = put(cps, 3 * (size_t)npanels);
+  g.normals = put(normals, 3 * (size_t)npanels);
+  g.cp_offset = put(cp_offset, (size_t)npanels);
+  int32_t* idx = reinterpret_cast<int32_t*>(at);
+  g.offsets = idx;
+  g.pnodes = idx + npanels + 1;
+  FP_CUDA_TRY(c->err, cudaMemcpyAsync(idx, offsets, (npanels + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream));
+  FP_CUDA_TRY(c->err, cudaMemcpyAsync(idx + npanels + 1, pnodes, offsets[npanels] * sizeof(int32_t),
+                                      cudaMemcpyHostToDevice, c->stream));
+  FP_CUDA_TRY(c->err, cudaGetLastError());
+  if (int rc = launch_geometry(c, g)) return rc;
+  c->h_tgt_valid = false;
+  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));   // the caller may change its arrays (pinned ones too)
   c->has_geometry = true;
   c->nsh = 0;
   c->h_shed.clear();
@@ -1355,6 +1308,7 @@ int fp_assembly_vjp(fp_ctx* c, const double* lambda, const double* gamma, const 
   c->kms[FP_STAGE_VJP] = ms;
   // residual r = b - A Gamma with b_i = -Uinf_i . n_i: d(lambda^T r)/dn_i =
   // -lambda_i (U_i + Uinf_i), d/dUinf_i = -lambda_i n_i, d/dX_i from the kernel
+  if (int rc = host_targets(c)) return rc;
   const double* T = c->h_tgt.data();
   for (int64_t i = 0; i < n; ++i) {
     for (int d = 0; d < 3; ++d) {

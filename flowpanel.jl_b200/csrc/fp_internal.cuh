@@ -73,12 +73,15 @@ struct fp_ctx {
   std::vector<double> h_nodes;
   std::vector<int32_t> h_shed;
   std::vector<double> h_Da, h_Db;
-  std::vector<double> h_tgt;            // 6 x N SoA copy of d_tgt
+  std::vector<double> h_tgt;            // 6 x N SoA copy of d_tgt, made when a call first needs it
+  bool h_tgt_valid = false;
 
   // device buffers
   fpb::PanelRec* d_panels = nullptr;    // N records
   fpb::SourceRec* d_src = nullptr;      // N records (source bodies)
   double* d_tgt = nullptr;              // 6 x N SoA: cx, cy, cz, nx, ny, nz
+  double* d_geo = nullptr;              // the arrays of fp_set_geometry as they came
+  size_t cap_geo = 0;                   // doubles
   WakeRec* d_wake = nullptr;            // nsh records
   double* d_G = nullptr;                // FP64 AIC, ld x N
   double* d_LU = nullptr;               // FP64 factors, ld x N
@@ -226,6 +229,15 @@ struct fp_ctx {
 };
 
 namespace fpb {
+
+// panel records and targets from the caller's mesh (fp_geometry.cu); null cps /
+// normals are formed as the reference does, cp_offset null is 1e-14
+struct GeometryArgs {
+  const double *nodes, *cps, *normals, *cp_offset;
+  const int32_t *offsets, *pnodes;
+};
+int launch_geometry(fp_ctx* c, const GeometryArgs& g);
+int host_targets(fp_ctx* c);   // c->h_tgt holds d_tgt
 
 // assembly (fp_assembly.cu)
 int launch_assemble_ring(fp_ctx* c, double offset, double cutoff, bool write32, cudaStream_t s = nullptr);

@@ -899,6 +899,7 @@ int fp_surface_loads(fp_ctx* c, int element, const double* strengths, const doub
   double* d_kw = d_nodal + nn;
   double* d_lds = d_kw + c->nkcell;
   double* d_hats = d_lds + 9;
+  if (int rc = host_targets(c)) return rc;
   std::vector<double> sg, cps(3 * N);
   signs_of(cp_offset, N, sg);
   for (int64_t i = 0; i < N; ++i)
