@@ -98,6 +98,8 @@ void free_matrices(fp_ctx* c) {
   if (c->d_minv) { cudaFree(c->d_minv); c->d_minv = nullptr; }
   dfree(c->d_rhs); dfree(c->d_x); dfree(c->d_r); dfree(c->d_w32); dfree(c->d_norms);
   dfree(c->d_V); dfree(c->d_h);
+  if (c->h_gm) cudaFreeHost(c->h_gm);
+  c->h_gm = nullptr;
   dfree(c->d_ab); dfree(c->d_ax); dfree(c->d_ar); dfree(c->d_aw32); dfree(c->d_anorms);
   c->cap_adj = 0;
   dfree(c->d_vjp);
@@ -187,6 +189,8 @@ int fp_ctx_destroy(fp_ctx* c) {
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->ktimer.pool) cudaEventDestroy(e);
   for (cudaEvent_t e : c->trace.pool) cudaEventDestroy(e);
+  for (cudaEvent_t e : c->ev_gm)
+    if (e) cudaEventDestroy(e);
   if (c->ev_panel) cudaEventDestroy(c->ev_panel);
   if (c->ev_rest) cudaEventDestroy(c->ev_rest);
   if (c->ev_g64) cudaEventDestroy(c->ev_g64);

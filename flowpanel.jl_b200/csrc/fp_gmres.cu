@@ -7,7 +7,16 @@
 // dot products and updates per step instead of j sequential MGS steps); the
 // small Hessenberg least-squares problem (Givens rotations) runs on the host.
 // Stop test as Krylov.jl: the residual estimate <= atol + rtol ||r0||.
+//
+// A step is seven short kernels (A v is HBM-bound: 8 N^2 bytes; the others are
+// latency-bound), launched programmatically dependent. Nothing of it waits for
+// the host: the last kernel normalises V_{j+1} and leaves column j of the
+// Hessenberg matrix in mapped host memory, and the host, which only decides
+// when to stop, runs its rotations kAhead steps behind the launches. 252 steps at
+// N = 3,828 (A, 117 MB, about fills L2): 39 us a step, of which A v 23; with a
+// host synchronisation and plain loads a step took 236 us.
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "fp_internal.cuh"
@@ -16,13 +25,46 @@ namespace fpb {
 
 constexpr int kDotThreads = 256;
 
-// h[i] = V_i . w, i < nv
-__global__ void k_dots(const double* __restrict__ V, int64_t ld, int nv, const double* __restrict__ w,
-                       int64_t n, double* __restrict__ h) {
+// What these passes move is small (4 MB of basis vectors, or the matrix from L2
+// and HBM), so memory latency over the bytes in flight is what they take; plain
+// loads were scheduled one or two ahead of their use whatever the source said
+// (A v 33 to 68 us at N = 3,828, the projections 19 to 29). So every operand is
+// copied to shared memory by cp.async, all of it in flight at once, and summed
+// from there, in the order of the plain loops.
+//
+// The step's kernels start before the previous one has ended (griddep_wait), so
+// what that one writes is read only after it.
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// a[0 .. count) -> dst, count rounded up to whole 16 bytes (the vectors' leading dimension is even)
+__device__ __forceinline__ void stage(double* dst, const double* a, int count) {
+  for (int q = 2 * threadIdx.x; q < count; q += 2 * blockDim.x) cp16(dst + q, a + q);
+}
+
+// h[i] = V_i . w, i < nv: one CTA a vector, 4,096 rows staged at a time
+constexpr int kDotRows = 4096;
+__global__ void __launch_bounds__(kDotThreads)
+k_dots(const double* V, int64_t ld, int nv, const double* w, int64_t n, double* h) {
+  extern __shared__ __align__(16) double st[];
   __shared__ double red[kDotThreads / 32];
+  griddep_wait();
+  griddep_launch();
   const int i = blockIdx.x;
   double s = 0.0;
-  for (int64_t r = threadIdx.x; r < n; r += kDotThreads) s += V[(int64_t)i * ld + r] * w[r];
+  for (int64_t r0 = 0; r0 < n; r0 += kDotRows) {
+    const int m = (int)imin64(kDotRows, n - r0);
+    __syncthreads();
+    stage(st, V + (int64_t)i * ld + r0, m);
+    stage(st + kDotRows, w + r0, m);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    for (int r = threadIdx.x; r < m; r += kDotThreads) s += st[r] * st[kDotRows + r];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
@@ -34,14 +76,132 @@ __global__ void k_dots(const double* __restrict__ V, int64_t ld, int nv, const d
   }
 }
 
-// w -= sum_i h[i] V_i ; acc[i] += h[i]
-__global__ void k_sub_Vh(const double* __restrict__ V, int64_t ld, int nv, const double* __restrict__ h,
-                         double* __restrict__ w, int64_t n) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= n) return;
-  double s = w[r];
-  for (int i = 0; i < nv; ++i) s -= h[i] * V[(int64_t)i * ld + r];
-  w[r] = s;
+// w -= sum_i h[i] V_i: 32 rows a CTA, 128 vectors staged at a time by 256
+// threads, the rows' chains by the first warp
+constexpr int kSubRows = 32, kSubVecs = 128, kSubThreads = 256;
+__global__ void __launch_bounds__(kSubThreads)
+k_sub_Vh(const double* V, int64_t ld, int nv, const double* h, double* w, int64_t n) {
+  extern __shared__ __align__(16) double st[];   // two of [vector][row], then the coefficients
+  griddep_wait();
+  griddep_launch();
+  const int64_t r0 = (int64_t)blockIdx.x * kSubRows, r = r0 + threadIdx.x;
+  const bool mine = threadIdx.x < kSubRows && r < n;
+  double* const sh = st + 2 * kSubVecs * kSubRows;
+  auto issue = [&](int i0) {
+    double* dst = st + ((i0 / kSubVecs) & 1) * kSubVecs * kSubRows;
+    for (int e = threadIdx.x; e < min(kSubVecs, nv - i0) * (kSubRows / 2); e += kSubThreads) {
+      const int i = e / (kSubRows / 2), q = 2 * (e % (kSubRows / 2));
+      cp16(dst + i * kSubRows + q, V + (int64_t)(i0 + i) * ld + r0 + q);   // ld is a multiple of 64
+    }
+    cp_commit();
+  };
+  issue(0);
+  double s = mine ? w[r] : 0.0;
+  for (int i0 = 0; i0 < nv; i0 += kSubVecs) {
+    const int m = min(kSubVecs, nv - i0);
+    if (i0 + kSubVecs < nv) { issue(i0 + kSubVecs); cp_wait<1>(); } else { cp_wait<0>(); }
+    if ((int)threadIdx.x < m) sh[threadIdx.x] = h[i0 + threadIdx.x];
+    __syncthreads();
+    const double* v = st + ((i0 / kSubVecs) & 1) * kSubVecs * kSubRows + threadIdx.x;
+    if (mine)
+#pragma unroll 8
+      for (int i = 0; i < m; ++i) s -= sh[i] * v[i * kSubRows];
+    __syncthreads();
+  }
+  if (mine) w[r] = s;
+}
+
+// parts of w = A v: 128 rows and one of kGemvSplitHost column ranges a CTA, 16
+// columns a stage; the first stages of A are under way before v is there
+constexpr int kMvRows = 128, kMvCols = 16, kMvStages = 3;   // four CTAs an SM: the grid of 3,828 rows in one wave
+constexpr size_t kMvSmem = (size_t)kMvStages * kMvCols * (kMvRows + 1) * sizeof(double);
+__global__ void __launch_bounds__(kMvRows)
+k_matvec(const double* __restrict__ A, int64_t lda, int64_t n, const double* v, double* part) {
+  extern __shared__ __align__(16) double st[];
+  double* const sv = st + kMvStages * kMvCols * kMvRows;   // v of each stage's columns
+  const int64_t i0 = (int64_t)blockIdx.x * kMvRows, i = i0 + threadIdx.x;
+  const int64_t cs = (n + gridDim.y - 1) / gridDim.y;
+  const int64_t c0 = blockIdx.y * cs, c1 = imin64(n, c0 + cs);
+  const int steps = c1 > c0 ? (int)((c1 - c0 + kMvCols - 1) / kMvCols) : 0;
+  const int rows = (int)imin64(kMvRows, lda - i0);
+  auto issue = [&](int t) {
+    if (t < steps) {
+      const int64_t j0 = c0 + (int64_t)t * kMvCols;
+      double* dst = st + (t % kMvStages) * kMvCols * kMvRows;
+#pragma unroll
+      for (int u = 0; u < kMvCols / 2; ++u) {   // 64 threads a column
+        const int e = threadIdx.x + u * kMvRows, c = e / (kMvRows / 2), q = 2 * (e % (kMvRows / 2));
+        if (j0 + c < c1 && q < rows) cp16(dst + c * kMvRows + q, A + (j0 + c) * lda + i0 + q);
+      }
+    }
+    cp_commit();
+  };
+#pragma unroll
+  for (int t = 0; t < kMvStages - 1; ++t) issue(t);
+  griddep_wait();
+  griddep_launch();
+  double s = 0.0;
+  for (int t = 0; t < steps; ++t) {
+    const int64_t j0 = c0 + (int64_t)t * kMvCols;
+    const int m = (int)imin64(kMvCols, c1 - j0);
+    double* const svt = sv + (t % kMvStages) * kMvCols;
+    if ((int)threadIdx.x < m) svt[threadIdx.x] = v[j0 + threadIdx.x];
+    cp_wait<kMvStages - 2>();
+    __syncthreads();   // stage t has landed; the one before it is read
+    issue(t + kMvStages - 1);
+    const double* a = st + (t % kMvStages) * kMvCols * kMvRows + threadIdx.x;
+    if (m == kMvCols) {
+#pragma unroll
+      for (int c = 0; c < kMvCols; ++c) s += a[c * kMvRows] * svt[c];
+    } else {
+      for (int c = 0; c < m; ++c) s += a[c * kMvRows] * svt[c];
+    }
+  }
+  cp_wait<0>();
+  if (i < n) part[blockIdx.y * n + i] = s;
+}
+__global__ void k_matvec_sum(const double* part, int64_t n, double* w) {
+  griddep_wait();
+  griddep_launch();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = 0.0;
+#pragma unroll
+  for (int p = 0; p < kGemvSplitHost; ++p) s += part[p * n + i];
+  w[i] = s;
+}
+
+// v_next = w / ||w|| (every CTA forms the norm), and to the host column j of the
+// Hessenberg matrix: h + h2, then ||w||
+__global__ void __launch_bounds__(kDotThreads)
+k_next(const double* w, int64_t n, double* v_next, const double* h, const double* h2, int nv, double* out) {
+  extern __shared__ __align__(16) double st[];
+  __shared__ double red[kDotThreads / 32];
+  griddep_wait();
+  griddep_launch();
+  double s = 0.0;
+  for (int64_t r0 = 0; r0 < n; r0 += kDotRows) {
+    const int m = (int)imin64(kDotRows, n - r0);
+    __syncthreads();
+    stage(st, w + r0, m);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    for (int r = threadIdx.x; r < m; r += kDotThreads) s += st[r] * st[r];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  double t = 0.0;
+  for (int q = 0; q < kDotThreads / 32; ++q) t += red[q];
+  const double norm = sqrt(t), alpha = 1.0 / norm;
+  const int64_t r = (int64_t)blockIdx.x * kDotThreads + threadIdx.x;
+  if (r < n) v_next[r] = alpha * w[r];
+  if (blockIdx.x == 0) {
+    for (int i = threadIdx.x; i < nv; i += kDotThreads) out[i] = h[i] + h2[i];
+    if (threadIdx.x == 0) out[nv] = norm;
+  }
 }
 
 // u = V y (nv columns)
@@ -101,13 +261,20 @@ struct Gm {
 
 // Device buffers for a basis of `cap` vectors: d_V holds the work vector w,
 // the correction u, then V_0 .. V_cap (cap + 3 columns of ld); d_h holds the
-// norms, two projection vectors of cap + 1 entries and y. `keep` columns of
-// the old basis (w and u included) are carried over when it grows.
+// norms, two projection vectors of cap + 1 entries and y; h_gm (mapped host
+// memory) the Hessenberg columns of kRing steps, cap + 2 entries each. `keep`
+// columns of the old basis (w and u included) and the columns the host has not
+// read yet are carried over when it grows.
+constexpr int kAhead = 2, kRing = kAhead + 1;
 int ensure_basis(fp_ctx* c, int cap, int keep) {
   if (c->cap_gmres_m >= cap) return FP_OK;
   const int64_t ld = c->ld;
   double* V = nullptr;
   double* h = nullptr;
+  double* ring = nullptr;
+  FP_CUDA_TRY(c->err, cudaHostAlloc(&ring, (size_t)kRing * (cap + 2) * sizeof(double), cudaHostAllocMapped));
+  for (cudaEvent_t& e : c->ev_gm)
+    if (!e) FP_CUDA_TRY(c->err, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   FP_CUDA_TRY(c->err, cudaMalloc(&V, (size_t)(cap + 3) * ld * sizeof(double)));
   FP_CUDA_TRY(c->err, cudaMalloc(&h, (size_t)(3 * (cap + 1) + 16) * sizeof(double)));
   if (c->d_V && keep > 0)
@@ -116,6 +283,12 @@ int ensure_basis(fp_ctx* c, int cap, int keep) {
   FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));
   if (c->d_V) cudaFree(c->d_V);
   if (c->d_h) cudaFree(c->d_h);
+  if (c->h_gm) {
+    const size_t old = (size_t)c->cap_gmres_m + 2;
+    for (int q = 0; q < kRing; ++q) std::memcpy(ring + q * (size_t)(cap + 2), c->h_gm + q * old, old * sizeof(double));
+    cudaFreeHost(c->h_gm);
+  }
+  c->h_gm = ring;
   c->d_V = V;
   c->d_h = h;
   c->cap_gmres_m = cap;
@@ -155,7 +328,7 @@ int gmres_solve(fp_ctx* c, const double* b, double* x, int64_t k, const fp_solve
   // host side of the Arnoldi process: column j of the rotated Hessenberg
   // matrix (j + 2 entries), the rotations and the rotated right-hand side
   std::vector<std::vector<double>> H;
-  std::vector<double> cs, sn, g, h, h2, y;
+  std::vector<double> cs, sn, g, y;
   for (int64_t q = 0; q < k; ++q) {
     const double* bq = b + q * ld;
     double* xq = x + q * ld;
@@ -180,55 +353,60 @@ int gmres_solve(fp_ctx* c, const double* b, double* x, int64_t k, const fp_solve
       g.assign(1, beta);
       int kd = 0;
       bool solved = false;
-      for (int j = 0; it < itmax; ++j) {
-        if (restart && j >= mem) break;
+      // launches of step j: w = A V_j (or A M^-1 V_j), orthogonalised twice,
+      // V_{j+1}, column j of the Hessenberg matrix to its slot of the ring
+      auto launch = [&](int j) -> int {
+        if (j + 1 > c->cap_gmres_m) {   // the basis outgrows its storage hint: room for V_{j+1}
+          const int cap2 = (int)std::min<int64_t>(2 * (int64_t)c->cap_gmres_m, itmax);
+          if (int rc = ensure_basis(c, std::max(cap2, j + 1), j + 3)) return rc;
+        }
         double* const w = c->d_V;
-        double* const u = c->d_V + ld;
         double* const V = c->d_V + 2 * ld;
         double* const dh = c->d_h + 8;
-        double* vj = V + (size_t)j * ld;
-        const double* src = vj;
+        double* const dh2 = dh + c->cap_gmres_m + 1;
+        const double* src = V + (size_t)j * ld;
         if (precondition) {
-          FP_CUDA_TRY(c->err, cudaMemcpyAsync(u, vj, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+          double* const u = c->d_V + ld;
+          FP_CUDA_TRY(c->err, cudaMemcpyAsync(u, src, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
           if (int rc = G.precond(u)) return rc;
           src = u;
         }
-        // w = A src  (residual form with b = 0: w = -(A src); negate via scale)
-        FP_CUDA_TRY(c->err, cudaMemsetAsync(c->d_r, 0, n * sizeof(double), c->stream));
-        if (int rc = gemv_residual(c, c->d_G, n, ld, src, c->d_r, w, 1)) return rc;
-        k_scale<<<G.g1, 256, 0, c->stream>>>(w, -1.0, w, n);
-        ++c->nlaunch;
-        // classical Gram-Schmidt, twice
-        h.resize(j + 1);
-        h2.resize(j + 1);
-        k_dots<<<j + 1, kDotThreads, 0, c->stream>>>(V, ld, j + 1, w, n, dh);
-        ++c->nlaunch;
-        k_sub_Vh<<<G.g1, 256, 0, c->stream>>>(V, ld, j + 1, dh, w, n);
-        ++c->nlaunch;
-        FP_CUDA_TRY(c->err, cudaMemcpyAsync(h.data(), dh, (j + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        k_dots<<<j + 1, kDotThreads, 0, c->stream>>>(V, ld, j + 1, w, n, dh + c->cap_gmres_m + 1);
-        ++c->nlaunch;
-        k_sub_Vh<<<G.g1, 256, 0, c->stream>>>(V, ld, j + 1, dh + c->cap_gmres_m + 1, w, n);
-        ++c->nlaunch;
-        FP_CUDA_TRY(c->err, cudaMemcpyAsync(h2.data(), dh + c->cap_gmres_m + 1, (j + 1) * sizeof(double), cudaMemcpyDeviceToHost,
-                                            c->stream));
-        double hn2 = 0;
-        if (int rc = G.norm2(w, &hn2)) return rc;   // syncs the stream
-        const double hn = std::sqrt(hn2);
+        const dim3 gm((unsigned)((n + kMvRows - 1) / kMvRows), kGemvSplitHost);
+        const unsigned gs = (unsigned)((n + kSubRows - 1) / kSubRows);
+        constexpr size_t sm_dot = 2 * kDotRows * sizeof(double), sm_next = kDotRows * sizeof(double),
+                         sm_sub = (size_t)(2 * kSubRows + 1) * kSubVecs * sizeof(double);
+        static SmemAttr am, ad, as;
+        FP_CUDA_TRY(c->err, am.ensure(k_matvec, (int)kMvSmem));
+        FP_CUDA_TRY(c->err, ad.ensure(k_dots, (int)sm_dot));
+        FP_CUDA_TRY(c->err, as.ensure(k_sub_Vh, (int)sm_sub));
+        launch_k(true, k_matvec, gm, dim3(kMvRows), kMvSmem, c->stream, c->d_G, ld, n, src, c->d_part);
+        launch_k(true, k_matvec_sum, dim3(G.g1), dim3(256), 0, c->stream, c->d_part, n, w);
+        for (double* hq : {dh, dh2}) {   // classical Gram-Schmidt, twice
+          launch_k(true, k_dots, dim3(j + 1), dim3(kDotThreads), sm_dot, c->stream, V, ld, j + 1, w, n, hq);
+          launch_k(true, k_sub_Vh, dim3(gs), dim3(kSubThreads), sm_sub, c->stream, V, ld, j + 1, hq, w, n);
+        }
+        launch_k(true, k_next, dim3(G.g1), dim3(kDotThreads), sm_next, c->stream, w, n, V + (size_t)(j + 1) * ld, dh, dh2,
+                 j + 1, c->h_gm + (size_t)(j % kRing) * (c->cap_gmres_m + 2));
+        c->nlaunch += 7;
+        FP_CUDA_TRY(c->err, cudaGetLastError());
+        FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_gm[j % kRing], c->stream));
+        return FP_OK;
+      };
+      // a preconditioned step is a whole solve: none is launched in vain
+      const int ahead = precondition ? 0 : kAhead;
+      const int64_t steps = std::min<int64_t>(restart ? mem : itmax, itmax - it);
+      int queued = 0;
+      for (int j = 0; j < steps; ++j) {
+        for (; queued <= j + ahead && queued < steps; ++queued)
+          if (int rc = launch(queued)) return rc;
+        FP_CUDA_TRY(c->err, cudaEventSynchronize(c->ev_gm[j % kRing]));
+        const double* hj = c->h_gm + (size_t)(j % kRing) * (c->cap_gmres_m + 2);
+        const double hn = hj[j + 1];
         H.emplace_back(j + 2);
         std::vector<double>& Hj = H.back();
-        for (int i = 0; i <= j; ++i) Hj[i] = h[i] + h2[i];
+        for (int i = 0; i <= j; ++i) Hj[i] = hj[i];
         Hj[j + 1] = hn;
         const bool breakdown = hn <= btol;
-        if (!breakdown) {
-          if (j + 1 > c->cap_gmres_m) {   // the basis outgrows its storage hint: room for V_{j+1}
-            const int cap2 = (int)std::min<int64_t>(2 * (int64_t)c->cap_gmres_m, itmax);
-            if (int rc = ensure_basis(c, std::max(cap2, j + 1), j + 3)) return rc;
-          }
-          k_scale<<<G.g1, 256, 0, c->stream>>>(c->d_V, 1.0 / hn, c->d_V + 2 * ld + (size_t)(j + 1) * ld, n);
-          ++c->nlaunch;
-        }
-        FP_CUDA_TRY(c->err, cudaGetLastError());
         // Givens rotations
         for (int i = 0; i < j; ++i) {
           const double t = cs[i] * Hj[i] + sn[i] * Hj[i + 1];

@@ -147,6 +147,8 @@ struct fp_ctx {
   double* d_V = nullptr;                // (m+1) x ld Krylov basis
   double* d_h = nullptr;                // small vectors
   int cap_gmres_m = 0;
+  double* h_gm = nullptr;               // mapped host memory: the Hessenberg columns of the steps under way
+  cudaEvent_t ev_gm[3] = {nullptr, nullptr, nullptr};
 
   // timing
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
