@@ -92,6 +92,8 @@ void free_matrices(fp_ctx* c) {
   c->g64_pending = false;
   dfree(c->d_G); dfree(c->d_LU); dfree(c->d_G32); dfree(c->d_ipiv);
   dfree(c->d_dinv64); dfree(c->d_dinv32); dfree(c->d_flags); dfree(c->d_mbox); dfree(c->d_part);
+  dfree(c->d_res);
+  c->cap_res = 0;
   dfree(c->d_dinv128_64); dfree(c->d_dinv128_32); dfree(c->d_mprev64); dfree(c->d_mprev32);
   dfree(c->d_mq32); dfree(c->d_ms32); dfree(c->d_zbox);
   c->trs2_ready = false;

@@ -122,6 +122,8 @@ struct fp_ctx {
   bool pdiag_linv = false;              // static-order LU: k_pdiag forms the full inv(L), no k_pinv (FP_TUNE_PDIAG_LINV)
   bool trs2_ready = false;              // R and S formed for the current FP32 factors
   double* d_part = nullptr;             // GEMV partial sums
+  double* d_res = nullptr;              // partial sums of the residual of several right-hand sides
+  size_t cap_res = 0;                   // doubles
   void* d_minv = nullptr;               // per block of a panel: M' = inv(L11) P11 (NB x NB, FP64 size), then the row order (NB ints)
   double* d_norms = nullptr;            // column norms (2 x cap_rhs)
   int64_t cap_rhs = 0;                  // allocated RHS columns
@@ -259,6 +261,10 @@ int gemm_sub_f64(fp_ctx* c, const double* A, const double* B, double* C, int64_t
 template <class T>
 int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv, T* B,
              int64_t ldb, int64_t k, bool transpose);
+// several right-hand sides at once (fp_trsm.cu)
+template <class T>
+int trsm_sweeps(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const T* D128, const T* Mp, T* B, int64_t ldb, int64_t k);
+int resid_multi(fp_ctx* c, const double* A, int64_t n, int64_t lda, const double* x, const double* b, double* r, int64_t k);
 int gemv_residual(fp_ctx* c, const double* A, int64_t n, int64_t lda, const double* x,
                   const double* b, double* r, int64_t k);
 // r = b - A^T x (FP64); x, b, r share the leading dimension lda

@@ -1958,14 +1958,14 @@ static int run_trs(fp_ctx* c, const T* A, int64_t n, int64_t lda, const T* Dinv,
   return FP_OK;
 }
 
-template <class T, bool TRANS = false>
+template <class T>
 static int solve_group(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const T* Dinv, T* B,
                        int64_t ldb, int kr) {
   int rc;
 #define FP_TRS_CASE(KR)                                                               \
   case KR:                                                                            \
-    if ((rc = run_trs<T, true, KR, TRANS>(c, LU, n, lda, Dinv, B, ldb))) return rc;   \
-    return run_trs<T, false, KR, TRANS>(c, LU, n, lda, Dinv, B, ldb);
+    if ((rc = run_trs<T, true, KR, true>(c, LU, n, lda, Dinv, B, ldb))) return rc;    \
+    return run_trs<T, false, KR, true>(c, LU, n, lda, Dinv, B, ldb);
   switch (kr) {
     FP_TRS_CASE(1)
     FP_TRS_CASE(2)
@@ -1990,7 +1990,7 @@ int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv
     for (int64_t q0 = 0; q0 < k;) {
       const int64_t left = k - q0;
       const int kr = left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
-      int rc = solve_group<T, true>(c, LU, n, lda, Dinv, B + q0 * ldb, ldb, kr);
+      int rc = solve_group<T>(c, LU, n, lda, Dinv, B + q0 * ldb, ldb, kr);
       if (rc) return rc;
       q0 += kr;
     }
@@ -2007,9 +2007,11 @@ int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv
     ++c->nlaunch;
     FP_CUDA_TRY(c->err, cudaGetLastError());
   }
-  if (k == 1) {   // one right-hand side: the 128-row streaming sweeps
-    const T* D128 = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_dinv128_64 : (void*)c->d_dinv128_32);
-    const T* Mp = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_mprev64 : (void*)c->d_mprev32);
+  const T* D128 = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_dinv128_64 : (void*)c->d_dinv128_32);
+  const T* Mp = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_mprev64 : (void*)c->d_mprev32);
+  // one right-hand side, or two in turn: the 128-row streaming sweeps (FP64, n =
+  // 12,000: 0.53 ms each against 1.58 ms for k_trsm's least group)
+  if (k <= 2) {
     static SmemAttr attr_lo, attr_up;
     FP_CUDA_TRY(c->err, attr_lo.ensure(k_trs1<T, true>, (int)trs1_smem<T>()));
     FP_CUDA_TRY(c->err, attr_up.ensure(k_trs1<T, false>, (int)trs1_smem<T>()));
@@ -2018,17 +2020,13 @@ int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv
       FP_CUDA_TRY(c->err, attr_lo2.ensure(k_trs1<float, true, true>, (int)trs1_smem<T>()));
       FP_CUDA_TRY(c->err, attr_up2.ensure(k_trs1<float, false, true>, (int)trs1_smem<T>()));
     }
-    if (int rc = run_trs1<T, true>(c, LU, n, lda, D128, Mp, B)) return rc;
-    return run_trs1<T, false>(c, LU, n, lda, D128, Mp, B);
+    for (int64_t q = 0; q < k; ++q) {
+      if (int rc = run_trs1<T, true>(c, LU, n, lda, D128, Mp, B + q * ldb)) return rc;
+      if (int rc = run_trs1<T, false>(c, LU, n, lda, D128, Mp, B + q * ldb)) return rc;
+    }
+    return FP_OK;
   }
-  for (int64_t q0 = 0; q0 < k;) {
-    const int64_t left = k - q0;
-    const int kr = left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
-    int rc = solve_group<T>(c, LU, n, lda, Dinv, B + q0 * ldb, ldb, kr);
-    if (rc) return rc;
-    q0 += kr;
-  }
-  return FP_OK;
+  return trsm_sweeps<T>(c, LU, n, lda, D128, Mp, B, ldb, k);
 }
 
 template <class T>
@@ -2105,6 +2103,7 @@ __global__ void k_gemv_finish(const double* __restrict__ part, int64_t n, const 
 
 int gemv_residual(fp_ctx* c, const double* A, int64_t n, int64_t lda, const double* x,
                   const double* b, double* r, int64_t k) {
+  if (k > 4) return resid_multi(c, A, n, lda, x, b, r, k);   // more than one pass over A by the groups below
   for (int64_t q0 = 0; q0 < k;) {
     const int64_t left = k - q0;
     const int kr = left >= 4 ? 4 : left >= 2 ? 2 : 1;
