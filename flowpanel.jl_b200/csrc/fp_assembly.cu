@@ -16,57 +16,31 @@ constexpr int kAsmPanels = 32;     // panels per CTA (smem tile)
 
 // HOT LOOP 1 of _G_Uvortexring! (src/FLOWPanel_liftingbody.jl:476-503): every
 // (control point, panel) pair. Targets on threads (coalesced column writes),
-// panel records staged in shared memory and broadcast to the CTA.
+// panel records staged in shared memory and broadcast to the CTA; nodes and
+// edges that consecutive panels share are evaluated once (fp_elements.cuh).
+// 12,000 panels with their wake: 2.40 -> 1.89 ms (1.95 with six blocks an SM);
+// with the straight-line reciprocals alone, 2.44: the FP64 pipe is what is busy.
 template <bool W32>
-__global__ void __launch_bounds__(kAsmThreads)
+__global__ void __launch_bounds__(kAsmThreads, 5)
 k_asm_ring(const PanelRec* __restrict__ panels, int64_t n, const double* __restrict__ tgt,
            int64_t ld, double offset, double cutoff2, double offset2, double* __restrict__ G,
            float* __restrict__ G32) {
-  __shared__ PanelRec sp[kAsmPanels];
-  __shared__ int quads;   // every panel of the tile has 4 nodes
+  __shared__ RingPanel<double> sp[kAsmPanels];
   const int64_t j0 = (int64_t)blockIdx.y * kAsmPanels;
   const int npt = (int)imin64(kAsmPanels, n - j0);
-  {
-    const double* src = reinterpret_cast<const double*>(panels + j0);
-    double* dst = reinterpret_cast<double*>(sp);
-    for (int q = threadIdx.x; q < npt * 16; q += kAsmThreads) dst[q] = src[q];
-  }
-  if (threadIdx.x < 32) {
-    const bool q4 = threadIdx.x >= npt || (int)panels[j0 + threadIdx.x].nn == 4;
-    const unsigned all = __all_sync(0xffffffffu, q4);
-    if (threadIdx.x == 0) quads = (int)all;
-  }
+  for (int q = threadIdx.x; q < npt * 16; q += kAsmThreads) stage_ring<double>(sp[q / 16], panels[j0 + q / 16], 1.0, q % 16);
   __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * kAsmThreads + threadIdx.x;
   if (i >= n) return;
   const double X = tgt[i], Y = tgt[n + i], Z = tgt[2 * n + i];
   const double n1 = tgt[3 * n + i], n2 = tgt[4 * n + i], n3 = tgt[5 * n + i];
-  if (quads) {
-    // two panels a step, no per-panel branch on the node count: the two
-    // entries' sqrt / reciprocal chains are independent and interleave
-    int jj = 0;
-    for (; jj + 1 < npt; jj += 2) {
-      const double g0 = ring_dot_n<double, 4>(sp[jj].p, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
-      const double g1 = ring_dot_n<double, 4>(sp[jj + 1].p, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
-      const int64_t idx = (j0 + jj) * ld + i;
-      G[idx] = g0;
-      G[idx + ld] = g1;
-      if (W32) {
-        G32[idx] = (float)g0;
-        G32[idx + ld] = (float)g1;
-      }
-    }
-    if (jj < npt) {
-      const double g = ring_dot_n<double, 4>(sp[jj].p, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
-      const int64_t idx = (j0 + jj) * ld + i;
-      G[idx] = g;
-      if (W32) G32[idx] = (float)g;
-    }
-    return;
-  }
+  RingNode<double> shared[2] = {};
+  double shared_edge = 0.0;
   for (int jj = 0; jj < npt; ++jj) {
-    const PanelRec& P = sp[jj];
-    const double g = ring_dot<double>(P.p, (int)P.nn, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
+    const RingPanel<double>& P = sp[jj];
+    const int link = jj > 0 ? P.link : 0, next = jj + 1 < npt ? sp[jj + 1].link : 0;
+    const double g = P.nn == 4 ? ring_walk_dot<4>(P, link, next, shared, shared_edge, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2)
+                               : ring_walk_dot<3>(P, link, next, shared, shared_edge, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
     const int64_t idx = (j0 + jj) * ld + i;
     G[idx] = g;
     if (W32) G32[idx] = (float)g;

@@ -18,7 +18,9 @@ constexpr double kFourPi = 4.0 * kPi;   // Julia's 4*pi (one rounding of the pro
 struct __align__(16) PanelRec {
   double p[12];   // node k at p[3k..3k+2]
   double nn;      // node count (3 or 4)
-  double pad[3];
+  int link;       // edge of the previous panel that edge 0 is, reversed (1..3), or 0 (fp_elements.cuh)
+  int pad0;
+  double pad[2];
 };
 
 // Error reporting: every entry point returns an FP_* status; the text of the

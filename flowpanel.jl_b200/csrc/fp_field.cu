@@ -12,11 +12,12 @@
 // few targets (the body's own control points) the panels are split in
 // gridDim.y chunks so that the grid fills the device: each chunk writes its
 // partial sum, the last chunk also the shedding edges, and k_uind_reduce adds
-// them to out in chunk order, in FP64. 100,000 probes of 36,600 panels in FP32:
-// 48.4 -> 22.8 ms with the straight-line reciprocals and four chunks (40 TF/s of
-// the operations counted above, 0.55 of the FP32 FMA peak; 2-norm error against
-// FP64 9.2e-6 -> 3.7e-6, the chunks' sums being shorter); 12,000 triangles at
-// their own control points in FP64: 3.1 -> 2.3 ms.
+// them to out in chunk order, in FP64. Panels of a strip share nodes and edges
+// (ring_walk). 100,000 probes of 36,600 panels in FP32: 48.4 -> 21.3 ms (22.8
+// without the sharing; the issue slots are 80 % busy, 168 instructions a panel
+// and warp; 2-norm error against FP64 9.2e-6 -> 3.7e-6, the chunks' sums being
+// shorter); 12,000 triangles at their own control points in FP64: 3.06 -> 1.60 ms
+// (1.66 with four blocks an SM instead of six).
 #include "fp_internal.cuh"
 
 namespace fpb {
@@ -25,12 +26,12 @@ constexpr int kFieldThreads = 128;
 constexpr int kFieldTile = 64;
 
 template <class T>
-__global__ void __launch_bounds__(kFieldThreads)
+__global__ void __launch_bounds__(kFieldThreads, sizeof(T) == 8 ? 6 : 8)
 k_uind_ring(const PanelRec* __restrict__ panels, const double* __restrict__ strength, int64_t n,
             const WakeRec* __restrict__ wake, int64_t nsh, const double* __restrict__ targets,
             int64_t m, double* __restrict__ out, double offset, double cutoff2, double offset2,
             double* __restrict__ partial) {
-  __shared__ __align__(16) T sp[kFieldTile][16];   // 12 coordinates, strength, node count; whole 16-byte loads
+  __shared__ RingPanel<T> sp[kFieldTile];
   const int64_t t = (int64_t)blockIdx.x * kFieldThreads + threadIdx.x;
   const bool live = t < m;
   const int64_t per = (n + gridDim.y - 1) / gridDim.y;
@@ -46,19 +47,10 @@ k_uind_ring(const PanelRec* __restrict__ panels, const double* __restrict__ stre
   for (int64_t j0 = jb; j0 < je; j0 += kFieldTile) {
     const int nt = (int)imin64(kFieldTile, je - j0);
     __syncthreads();
-    for (int q = threadIdx.x; q < nt * 16; q += kFieldThreads) {
-      const int jj = q / 16, e = q % 16;
-      const PanelRec& P = panels[j0 + jj];
-      sp[jj][e] = e == 12 ? (T)strength[j0 + jj] : e < 12 ? (T)P.p[e] : (T)P.nn;
-    }
+    for (int q = threadIdx.x; q < nt * 16; q += kFieldThreads)
+      stage_ring<T>(sp[q / 16], panels[j0 + q / 16], strength[j0 + q / 16], q % 16);
     __syncthreads();
-    if (live) {
-      for (int jj = 0; jj < nt; ++jj) {
-        const T* p = sp[jj];
-        if (p[13] == T(4)) ring_vel_n<T, 4>(p, p[12], X, Y, Z, off, c2, o2, u, v, w);
-        else ring_vel_n<T, 3>(p, p[12], X, Y, Z, off, c2, o2, u, v, w);
-      }
-    }
+    if (live) ring_walk<T>(sp, nt, X, Y, Z, off, c2, o2, u, v, w);
   }
   if (!live) return;
   for (int64_t e = 0; last && e < nsh; ++e) {

@@ -41,7 +41,13 @@ k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* 
 #pragma unroll
   for (int k = 0; k < 4; ++k) store3(r.p + 3 * k, P[k]);
   r.nn = nn;
-  r.pad[0] = r.pad[1] = r.pad[2] = 0.0;
+  r.link = r.pad0 = 0;
+  r.pad[0] = r.pad[1] = 0.0;
+  if (p > 0) {
+    const int q0 = a.offsets[p - 1], qn = o0 - q0;
+    for (int e = 1; e < qn; ++e)
+      if (a.pnodes[q0 + e] == a.pnodes[o0 + 1] && a.pnodes[q0 + (e + 1 == qn ? 0 : e + 1)] == a.pnodes[o0]) r.link = e;
+  }
   panels[p] = r;
 
   const V3 e = sub(P[1], P[0]), f = sub(P[2], P[0]);

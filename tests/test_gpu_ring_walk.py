@@ -1,0 +1,47 @@
+"""Consecutive panels that share an edge (ring_walk in fp_elements.cuh): every way
+the shared edge can lie, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _relabel(fp, m, turn):
+    """Each panel's nodes turned by `turn(panel)` places: another edge becomes edge 0."""
+    cells = [np.roll(m.panel(i), -turn(i)) for i in range(m.npanels)]
+    out = fp.meshes.Mesh(m.nodes.copy(), m.panel_offsets.copy(), np.concatenate(cells).astype(np.int32))
+    out.bodies = m.bodies
+    return out
+
+
+# turns that make edge 0 the shared one, or none of a run, or each edge of the
+# previous panel in turn; 130 quadrilaterals or 258 triangles: tiles of 32 and 64 with a rest
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("turn", [lambda i: 0, lambda i: 1, lambda i: 2, lambda i: i, lambda i: (i * i + i // 3)])
+def test_shared_edges(fp, O, split, turn):
+    s = fp.meshes.sphere(1.0, 12, 11)   # quadrilaterals, and triangles at the poles
+    m = fp.meshes.triangulate(s) if split else s
+    nn = np.diff(m.panel_offsets)
+    m = _relabel(fp, m, lambda i: turn(i) % nn[i])
+    body = fp.RigidWakeBody(m)
+    normals = fp.calc_normals(body)
+    cps = fp.calc_controlpoints(body, normals)
+    rng = np.random.default_rng(5)
+    g = rng.standard_normal(m.npanels)
+    X = np.concatenate([cps + 0.03 * normals, 3 * rng.standard_normal((67, 3)), m.nodes[:5]])   # and at nodes
+    c = fp._capi.Context(0)
+    try:
+        c.set_geometry(m.nodes, m.panel_offsets, m.panel_nodes, cps, normals)
+        c.assemble(fp._capi.FP_ELEMENT_VORTEXRING)
+        G = c.get_aic()
+        u64 = c.uind(fp._capi.FP_ELEMENT_VORTEXRING, g, X)
+        u32 = c.uind(fp._capi.FP_ELEMENT_VORTEXRING, g, X[:-5], None, fp._capi.FP_PREC_MIXED)
+    finally:
+        c.close()
+    none = np.zeros((0, 3))
+    Gr = O.assemble_vortexring(m, cps, normals, none, none)
+    assert np.abs(G - Gr).max() < 1e-12 * np.abs(Gr).max()
+    ur = O.uind_vortexring(m, g, none, none, X)
+    assert np.abs(u64 - ur).max() < 1e-12 * np.abs(ur).max()
+    # FP32: coordinates to 6e-8 of 1, distances from 0.03 on, sums of 130 to 258 panels
+    assert np.abs(u32 - ur[:-5]).max() < 1e-4 * np.abs(ur[:-5]).max()
