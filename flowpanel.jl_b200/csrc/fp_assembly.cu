@@ -34,7 +34,7 @@ k_asm_ring(const PanelRec* __restrict__ panels, int64_t n, const double* __restr
   if (i >= n) return;
   const double X = tgt[i], Y = tgt[n + i], Z = tgt[2 * n + i];
   const double n1 = tgt[3 * n + i], n2 = tgt[4 * n + i], n3 = tgt[5 * n + i];
-  RingNode<double> shared[2] = {};
+  RingNode shared[2] = {};
   double shared_edge = 0.0;
   for (int jj = 0; jj < npt; ++jj) {
     const RingPanel<double>& P = sp[jj];

@@ -12,12 +12,13 @@
 // few targets (the body's own control points) the panels are split in
 // gridDim.y chunks so that the grid fills the device: each chunk writes its
 // partial sum, the last chunk also the shedding edges, and k_uind_reduce adds
-// them to out in chunk order, in FP64. Panels of a strip share nodes and edges
-// (ring_walk). 100,000 probes of 36,600 panels in FP32: 48.4 -> 21.3 ms (22.8
-// without the sharing; the issue slots are 80 % busy, 168 instructions a panel
-// and warp; 2-norm error against FP64 9.2e-6 -> 3.7e-6, the chunks' sums being
-// shorter); 12,000 triangles at their own control points in FP64: 3.06 -> 1.60 ms
-// (1.66 with four blocks an SM instead of six).
+// them to out in chunk order, in FP64. Panels of a strip share nodes and, in
+// FP64, edges (ring_walk). Bound by instruction issue in FP32 and by the FP64 pipe.
+// 100,000 probes of 36,600 panels in FP32: 48.4 -> 26.4 ms, with the same bits
+// (33.3 without the step of two quadrilaterals; 27.0 with eight blocks an SM and
+// 26.7 with six instead of seven; 28.3 with 96 threads a block, 29.4 with 64).
+// 12,000 triangles at their own control points in FP64: 3.06 -> 1.60 ms (1.66
+// with four blocks an SM instead of six).
 #include "fp_internal.cuh"
 
 namespace fpb {
@@ -26,7 +27,7 @@ constexpr int kFieldThreads = 128;
 constexpr int kFieldTile = 64;
 
 template <class T>
-__global__ void __launch_bounds__(kFieldThreads, sizeof(T) == 8 ? 6 : 8)
+__global__ void __launch_bounds__(kFieldThreads, sizeof(T) == 8 ? 6 : 7)
 k_uind_ring(const PanelRec* __restrict__ panels, const double* __restrict__ strength, int64_t n,
             const WakeRec* __restrict__ wake, int64_t nsh, const double* __restrict__ targets,
             int64_t m, double* __restrict__ out, double offset, double cutoff2, double offset2,
@@ -44,13 +45,15 @@ k_uind_ring(const PanelRec* __restrict__ panels, const double* __restrict__ stre
   T v = live && !partial ? (T)out[3 * t + 1] : T(0);
   T w = live && !partial ? (T)out[3 * t + 2] : T(0);
   const T off = (T)offset, c2 = (T)cutoff2, o2 = (T)offset2;
+  const bool usual = sizeof(T) == 8 || ordinary_offsets((float)off, (float)c2, (float)o2);
   for (int64_t j0 = jb; j0 < je; j0 += kFieldTile) {
     const int nt = (int)imin64(kFieldTile, je - j0);
+    bool near = true;
     __syncthreads();
     for (int q = threadIdx.x; q < nt * 16; q += kFieldThreads)
-      stage_ring<T>(sp[q / 16], panels[j0 + q / 16], strength[j0 + q / 16], q % 16);
-    __syncthreads();
-    if (live) ring_walk<T>(sp, nt, X, Y, Z, off, c2, o2, u, v, w);
+      near = stage_ring<T>(sp[q / 16], panels[j0 + q / 16], strength[j0 + q / 16], q % 16) && near;
+    const bool ordinary = __syncthreads_and(near) && fabs(X) < T(0x1p20) && fabs(Y) < T(0x1p20) && fabs(Z) < T(0x1p20) && usual;
+    if (live) ring_walk(sp, nt, ordinary, X, Y, Z, off, c2, o2, u, v, w);
   }
   if (!live) return;
   for (int64_t e = 0; last && e < nsh; ++e) {
@@ -109,10 +112,11 @@ k_uind_reduce(const double* __restrict__ partial, int nchunk, int64_t m, double*
 }
 
 // Panel chunks for m targets: enough blocks for sixteen per SM, so that the last
-// ones to finish are a small part, chunks of at least 512 panels, at most 16.
-int uind_chunks(int64_t m, int64_t n) {
+// ones to finish are a small part, chunks of at least 512 panels, at most 16. In
+// FP32, where the chunks are part of the result, four per SM.
+int uind_chunks(int64_t m, int64_t n, bool fp32) {
   const int64_t blocks = (m + kFieldThreads - 1) / kFieldThreads;
-  const int64_t want = 16 * (int64_t)num_sms();
+  const int64_t want = (fp32 ? 4 : 16) * (int64_t)num_sms();
   if (blocks >= want) return 1;
   int64_t s = (want + blocks - 1) / blocks;
   s = imin64(s, imin64(16, n / 512));
@@ -174,7 +178,7 @@ int launch_phi(fp_ctx* c, const double* d_sigma, const double* d_mu, const doubl
 
 int launch_uind_ring(fp_ctx* c, const double* d_strength, const double* d_targets, int64_t m,
                      double* d_out, bool fp32) {
-  const int nchunk = uind_chunks(m, c->N);
+  const int nchunk = uind_chunks(m, c->N, fp32);
   if (nchunk > 1 && ensure_uind_scratch(c, (size_t)nchunk * 3 * m)) return FP_ECUDA;
   double* part = nchunk > 1 ? c->d_uscr : nullptr;
   const dim3 g((unsigned)((m + kFieldThreads - 1) / kFieldThreads), nchunk);
@@ -192,7 +196,7 @@ int launch_uind_ring(fp_ctx* c, const double* d_strength, const double* d_target
 
 int launch_uind_source(fp_ctx* c, const double* d_strength, const double* d_targets, int64_t m,
                        double* d_out) {
-  const int nchunk = uind_chunks(m, c->N);
+  const int nchunk = uind_chunks(m, c->N, false);
   if (nchunk > 1 && ensure_uind_scratch(c, (size_t)nchunk * 3 * m)) return FP_ECUDA;
   double* part = nchunk > 1 ? c->d_uscr : nullptr;
   const dim3 g((unsigned)((m + kFieldThreads - 1) / kFieldThreads), nchunk);
