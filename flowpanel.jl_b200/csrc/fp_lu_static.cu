@@ -27,7 +27,8 @@
 //               the split operands, with no separate split pass.
 // Look-ahead on two streams (lu_factor_static): the panel stream runs K1, K6,
 // then (after the previous panel's trailing update) K2 and K3 on the next
-// panel's columns; the second stream runs K2 and K5 on the columns beyond.
+// panel's columns; the second stream runs K2 and K5 on the columns beyond. Large systems
+// in the BF16-pair form go by groups of panels instead (lu_static_groups).
 // The panel width equals the triangular solves' 128-row blocks.
 #include <cuda_bf16.h>
 
@@ -536,7 +537,7 @@ constexpr size_t l21_smem() {
 template <int SM>
 __global__ void __launch_bounds__(L21_THREADS)
 k_l21(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int64_t rbeg, const float* __restrict__ dinv,
-      float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert) {
+      float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert, int ldo) {
   griddep_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   float (*X)[XP] = reinterpret_cast<float (*)[XP]>(smem);
@@ -608,7 +609,7 @@ k_l21(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int6
     const int r = e / C4, c = (e % C4) * 4;
     const float4 v = *reinterpret_cast<const float4*>(&X[r][c]);
     const float vv[4] = {v.x, v.y, v.z, v.w};
-    put_split<SM>(Ah, Al, (row0 - r0 + r) * (int64_t)PW + c, vv);
+    put_split<SM>(Ah, Al, (row0 - r0 + r) * (int64_t)ldo + c, vv);
     lmax = fmaxf(lmax, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
   }
 #pragma unroll
@@ -771,7 +772,7 @@ constexpr size_t l21a_smem() {
 template <int SM>
 __global__ void __launch_bounds__(L21_THREADS)
 k_l21a(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int64_t rbeg,
-       const float* __restrict__ dinv, float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert) {
+       const float* __restrict__ dinv, float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert, int ldo) {
   griddep_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   float (*XT)[XTP] = reinterpret_cast<float (*)[XTP]>(smem);
@@ -864,7 +865,7 @@ k_l21a(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int
     const int r = e % L21_ROWS, c = (e / L21_ROWS) * 4;
     if (r >= rows) continue;
     const float v[4] = {XT[c][r], XT[c + 1][r], XT[c + 2][r], XT[c + 3][r]};
-    put_split<SM>(Ah, Al, (row0 - r0 + r) * (int64_t)PW + c, v);
+    put_split<SM>(Ah, Al, (row0 - r0 + r) * (int64_t)ldo + c, v);
     lmax = fmaxf(lmax, fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
   }
 #pragma unroll
@@ -1036,7 +1037,7 @@ struct U12gCfg {
 template <int CW, int SM, bool DIAG = false>
 __global__ void __launch_bounds__(U12gCfg<CW>::THREADS)
 k_u12g(float* __restrict__ A, int64_t lda, int64_t k, int64_t c0, int64_t c1, const float* __restrict__ slot,
-       float* __restrict__ Bh, float* __restrict__ Bl, int64_t kd, int zasync) {
+       float* __restrict__ Bh, float* __restrict__ Bl, int64_t kd, int zasync, int ldo) {
   griddep_wait();
   typedef U12gCfg<CW> Cfg;
   constexpr int T = Cfg::THREADS, ZP = Cfg::ZP, CQ = CW / 4;
@@ -1101,7 +1102,7 @@ k_u12g(float* __restrict__ A, int64_t lda, int64_t k, int64_t c0, int64_t c1, co
     if (cb + b >= cols) break;
     const float v[4] = {acc[0][b], acc[1][b], acc[2][b], acc[3][b]};
     *reinterpret_cast<float4*>(A + (col0 + cb + b) * lda + k + ib) = make_float4(v[0], v[1], v[2], v[3]);
-    put_split<SM>(Bh, Bl, (col0 - c0 + cb + b) * (int64_t)PW + ib, v);
+    put_split<SM>(Bh, Bl, (col0 - c0 + cb + b) * (int64_t)ldo + ib, v);
   }
   if constexpr (DIAG) {
     __syncthreads();   // every warp is done with inv(L) and the A12 block
@@ -1144,6 +1145,151 @@ __global__ void k_iota(int32_t* __restrict__ ipiv, int64_t n) {
 }
 
 }  // namespace st
+
+// The factorisation by groups of G panels: the trailing update takes all the
+// group's 128 G columns at once, so that the matrix is read and written once per
+// group instead of once per panel, which bounds the update: at 128 columns the
+// passes over C take four times its MMAs, at 512 about as long. Within a group each panel's columns and rows
+// are updated by the panels before it only when their turn comes; after its last
+// panel, the next group's columns and rows come first, and the next group's panels
+// run beside the rest of the update. With panel p of the group at columns
+// [k, k1), k2 the end of the next one, F the group's end and H the next group's:
+//   stream   the chain of diagonal blocks: K1, K6 on rows [k1, k2), K2 on columns
+//            [k1, k2), update of the tile [k1, k2) x [k1, k2)
+//   stream3  inv(L); K6 on the rows from k2 on, then their update in the next
+//            panel's columns (after the last panel: in [F, H))
+//   stream4  K2 on the columns from k2 on, then their update in the next panel's
+//            rows (after the last panel: also in the rows up to H)
+//   stream2  after the last panel: [H, n) x [H, n)
+// The split operands hold the group's 128 G K values a row; rows and columns count
+// from the first panel's end. Their sets alternate by group.
+template <int G>
+static int lu_static_groups(fp_ctx* c, float* A, int64_t n, int64_t lda, float* cert) {
+  using namespace st;
+  typedef __nv_bfloat16 bf;
+  constexpr int LD = G * PW;
+  static_assert((size_t)LD * sizeof(bf) <= (size_t)kOuterPanel * sizeof(float), "a row of the split operands fits the scratch");
+  float* const dinv_base = reinterpret_cast<float*>(c->d_minv);
+  const auto at = [&](int64_t r, int64_t col) { return A + col * lda + r; };
+  const auto wait = [&](cudaStream_t s, cudaEvent_t e) { return cudaStreamWaitEvent(s, e, 0); };
+  const cudaStream_t s1 = c->stream, s2 = c->stream2, s3 = c->stream3, s4 = c->stream4;
+  for (cudaEvent_t e : {c->ev_rest, c->ev_tcr, c->ev_top}) FP_CUDA_TRY(c->err, cudaEventRecord(e, s1));
+  for (int64_t i = 0; i * PW < n; ++i) {
+    const int p = (int)(i % G), kk = (p + 1) * PW, set = (int)((i / G) & 1);
+    const bool last = p == G - 1;
+    const int64_t k = i * PW, base = k - p * PW;
+    const int64_t E = std::min<int64_t>(base + PW, n), k1 = std::min<int64_t>(k + PW, n), k2 = std::min<int64_t>(k + 2 * PW, n);
+    const int64_t H = std::min<int64_t>(base + 2 * LD, n);
+    float* const dinv = dinv_base + (size_t)(i & 1) * kSlotFloats;
+    bf* const op[4] = {reinterpret_cast<bf*>(c->d_tc[set][0]), reinterpret_cast<bf*>(c->d_tc[set][1]),
+                       reinterpret_cast<bf*>(c->d_tc[set][2]), reinterpret_cast<bf*>(c->d_tc[set][3])};
+    // C -= L21 U12 of the group's panels so far, on rows [r0, r1) and columns [q0, q1)
+    const auto update = [&](int64_t r0, int64_t r1, int64_t q0, int64_t q1) -> int {
+      if (r0 >= r1 || q0 >= q1) return FP_OK;
+      const int64_t ao = (r0 - E) * LD, bo = (q0 - E) * LD;
+      if (tc_gemm_sub_bf16x3(c, op[0] + ao, op[1] + ao, op[2] + bo, op[3] + bo, LD, at(r0, q0), lda, r1 - r0, q1 - q0, kk))
+        return FP_OK;
+      FP_CUDA_TRY(c->err, cudaGetLastError());
+      for (int64_t q = base; q < k1; q += PW)
+        if (int rc = gemm_sub_simt_f32(c, at(r0, q), at(q, q0), at(r0, q0), lda, r1 - r0, q1 - q0, PW)) return rc;
+      return FP_OK;
+    };
+    const auto l21 = [&](int64_t r0, int64_t r1) -> int {
+      if (r0 >= r1) return FP_OK;
+      TraceScope tr(c, TR_L21);
+      launch_k(c->pdl, k_l21a<kSplitBf16x2>, (unsigned)((r1 - r0 + L21_ROWS - 1) / L21_ROWS), L21_THREADS, l21a_smem(),
+               c->stream, A, lda, r1, k, E, r0, dinv, reinterpret_cast<float*>(op[0] + p * PW),
+               reinterpret_cast<float*>(op[1] + p * PW), cert, LD);
+      ++c->nlaunch;
+      FP_CUDA_TRY(c->err, cudaGetLastError());
+      return FP_OK;
+    };
+    const auto u12 = [&](int64_t q0, int64_t q1, bool narrow) -> int {
+      if (q0 >= q1) return FP_OK;
+      TraceScope tr(c, narrow ? TR_U12 : TR_STRIP);
+      float* const bh = reinterpret_cast<float*>(op[2] + (q0 - E) * LD + p * PW);
+      float* const bl = reinterpret_cast<float*>(op[3] + (q0 - E) * LD + p * PW);
+      const auto go = [&](auto kernel, int cw, int threads, size_t smem) {
+        launch_k(c->pdl, kernel, (unsigned)((q1 - q0 + cw - 1) / cw), threads, smem, c->stream, A, lda, k, q0, q1, dinv, bh, bl,
+                 (int64_t)0, (int)c->u12_async, LD);
+      };
+      if (narrow) go(k_u12g<16, kSplitBf16x2>, 16, U12gCfg<16>::THREADS, U12gCfg<16>::smem());
+      else if (c->u12_wide) go(k_u12g<64, kSplitBf16x2>, 64, U12gCfg<64>::THREADS, U12gCfg<64>::smem());
+      else go(k_u12g<32, kSplitBf16x2>, 32, U12gCfg<32>::THREADS, U12gCfg<32>::smem());
+      ++c->nlaunch;
+      FP_CUDA_TRY(c->err, cudaGetLastError());
+      return FP_OK;
+    };
+    // the chain. The slot of the inverses is free: what panel i - 2 left to the
+    // other streams came before the updates that panel i - 1 waited for
+    {
+      TraceScope tr(c, TR_DIAG);
+      launch_k(c->pdl, k_pdiag, 1, kDiagThreads, pdiag_smem(false), s1, A, lda, n, k, dinv, cert, c->d_status, (float*)nullptr);
+      ++c->nlaunch;
+      FP_CUDA_TRY(c->err, cudaGetLastError());
+    }
+    if (k1 == n) break;
+    FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_diag, s1));
+    {
+      OnStream on3(c, s3);
+      FP_CUDA_TRY(c->err, wait(s3, c->ev_diag));
+      TraceScope tr(c, TR_PINV);
+      launch_k(c->pdl, k_pinv, NIB, PI_THREADS, pinv_smem(), s3, A, lda, k, dinv);
+      ++c->nlaunch;
+      FP_CUDA_TRY(c->err, cudaGetLastError());
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_pinv, s3));
+    }
+    FP_CUDA_TRY(c->err, wait(s1, c->ev_tcr));   // this panel's rows from k1 on
+    if (int rc = l21(k1, k2)) return rc;
+    FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_panel, s1));
+    FP_CUDA_TRY(c->err, wait(s1, c->ev_top));   // its columns from k1 on
+    FP_CUDA_TRY(c->err, wait(s1, c->ev_pinv));
+    if (int rc = u12(k1, k2, true)) return rc;
+    FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_u12n, s1));
+    if (last) FP_CUDA_TRY(c->err, wait(s1, c->ev_rest));
+    if (int rc = update(k1, k2, k1, k2)) return rc;
+    if (k2 == n) continue;
+    {
+      OnStream on4(c, s4);   // U12 of the columns beyond
+      FP_CUDA_TRY(c->err, wait(s4, c->ev_pinv));
+      if (int rc = u12(k2, n, false)) return rc;
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_u12r, s4));
+    }
+    {
+      OnStream on3(c, s3);   // the rows below
+      if (int rc = l21(k2, n)) return rc;
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_l21t, s3));
+      FP_CUDA_TRY(c->err, wait(s3, c->ev_u12n));
+      if (last) {
+        FP_CUDA_TRY(c->err, wait(s3, c->ev_u12r));
+        FP_CUDA_TRY(c->err, wait(s3, c->ev_rest));
+      }
+      if (int rc = update(k2, n, k1, last ? H : k2)) return rc;
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_tcr, s3));
+    }
+    {
+      OnStream on4(c, s4);   // the columns beyond
+      FP_CUDA_TRY(c->err, wait(s4, c->ev_panel));
+      if (last) FP_CUDA_TRY(c->err, wait(s4, c->ev_rest));
+      if (int rc = update(k1, k2, k2, n)) return rc;
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_top, s4));
+      if (last && k2 < H && H < n) {
+        FP_CUDA_TRY(c->err, wait(s4, c->ev_l21t));
+        if (int rc = update(k2, H, H, n)) return rc;
+      }
+    }
+    if (last && H < n) {
+      OnStream on2(c, s2);
+      FP_CUDA_TRY(c->err, wait(s2, c->ev_u12r));
+      FP_CUDA_TRY(c->err, wait(s2, c->ev_l21t));
+      if (int rc = update(H, n, H, n)) return rc;
+      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, s2));
+    }
+  }
+  // the other streams' last work
+  for (cudaEvent_t e : {c->ev_rest, c->ev_tcr, c->ev_top, c->ev_pinv}) FP_CUDA_TRY(c->err, wait(s1, e));
+  return FP_OK;
+}
 
 // Host side of the look-ahead factorisation (see the head of this file). The
 // scratch: per panel parity, the 32 x 32 inverses (in c->d_minv) and the
@@ -1210,6 +1356,12 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
   FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
   if (c->rest_split) FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_top, c->stream));
   FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream2, c->ev_rest, 0));
+  // from 56 panels on by groups of four. Below, the chain of diagonal blocks bounds
+  // both forms (2,000 unknowns 0.97 ms, groups 0.98; 6,000 3.01, 3.06; 8,000 4.97,
+  // 4.40; 12,000 10.5, 8.1; 20,800 42.8, 24.6; 36,600 219, 113; groups of two: 4.58,
+  // 8.83, 30.9, 150; of three: 4.69, 8.63, 28.0, 131)
+  if (x3 && lside && !dl && c->lu_split && c->lu_overlap && !c->lu_fuse && !c->rest_split && c->l21_async && n >= 56 * PW)
+    return lu_static_groups<4>(c, A, n, lda, cert);
   // C -= L21 U12 on the rows [kend, n) and columns [cb, ce): tensor cores from
   // the split operands, or the SIMT kernel on the factors in place
   // (rows [kend + roff, kend + roff + mrows), mrows < 0: to n; roff rows into the L21 operand)
@@ -1303,10 +1455,10 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
         const int64_t he = kend + PW;   // the next panel's rows
         if (x3)
           launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16x2> : k_l21<kSplitBf16x2>, (unsigned)(PW / L21_ROWS), L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda,
-                   he, K0, kend, kend, dinv, s[0], s[1], cert);
+                   he, K0, kend, kend, dinv, s[0], s[1], cert, PW);
         else
           launch_k(c->pdl, c->l21_async ? k_l21a<kSplitTf32> : k_l21<kSplitTf32>, (unsigned)(PW / L21_ROWS), L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, he,
-                   K0, kend, kend, dinv, s[0], xsplit ? nullptr : al, cert);
+                   K0, kend, kend, dinv, s[0], xsplit ? nullptr : al, cert, PW);
         ++c->nlaunch;
         FP_CUDA_TRY(c->err, cudaGetLastError());
       }
@@ -1317,10 +1469,10 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
         const unsigned g = (unsigned)((n - kend - PW + L21_ROWS - 1) / L21_ROWS);
         if (x3)
           launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16x2> : k_l21<kSplitBf16x2>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend + PW,
-                   dinv, s[0], s[1], cert);
+                   dinv, s[0], s[1], cert, PW);
         else
           launch_k(c->pdl, c->l21_async ? k_l21a<kSplitTf32> : k_l21<kSplitTf32>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend + PW, dinv,
-                   s[0], xsplit ? nullptr : al, cert);
+                   s[0], xsplit ? nullptr : al, cert, PW);
         ++c->nlaunch;
         FP_CUDA_TRY(c->err, cudaGetLastError());
       }
@@ -1333,11 +1485,11 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
         if (x3) launch_k(c->pdl, k_l21g<kSplitBf16x2>, g, L21G_THREADS, l21g_smem(), c->stream, A, lda, n, K0, kend, dinv, s[0], s[1], cert);
         else launch_k(c->pdl, k_l21g<kSplitTf32>, g, L21G_THREADS, l21g_smem(), c->stream, A, lda, n, K0, kend, dinv, s[0], al, cert);
       } else if (bf16) {
-        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16> : k_l21<kSplitBf16>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], al, cert);
+        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16> : k_l21<kSplitBf16>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], al, cert, PW);
       } else if (x3) {
-        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16x2> : k_l21<kSplitBf16x2>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], s[1], cert);
+        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitBf16x2> : k_l21<kSplitBf16x2>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], s[1], cert, PW);
       } else {
-        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitTf32> : k_l21<kSplitTf32>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], al, cert);
+        launch_k(c->pdl, c->l21_async ? k_l21a<kSplitTf32> : k_l21<kSplitTf32>, g, L21_THREADS, c->l21_async ? l21a_smem() : l21_smem(), c->stream, A, lda, n, K0, kend, kend, dinv, s[0], al, cert, PW);
       }
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
@@ -1358,20 +1510,20 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
         const unsigned g = (unsigned)((knext - kend + 15) / 16);
         if (x3)
           launch_k(c->pdl, k_u12g<16, kSplitBf16x2, true>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend,
-                   knext, dinv, s[2], s[3], kend, (int)c->u12_async);
+                   knext, dinv, s[2], s[3], kend, (int)c->u12_async, PW);
         else
           launch_k(c->pdl, k_u12g<16, kSplitTf32, true>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend,
-                   knext, dinv, s[2], xsplit ? nullptr : s[3], kend, (int)c->u12_async);
+                   knext, dinv, s[2], xsplit ? nullptr : s[3], kend, (int)c->u12_async, PW);
         ++c->nlaunch;
         FP_CUDA_TRY(c->err, cudaGetLastError());
       } else {
         TraceScope tr(c, TR_U12);
         const unsigned g = (unsigned)((knext - kend + 15) / 16);
         if (x3)
-          launch_k(c->pdl, k_u12g<16, kSplitBf16x2>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2], s[3], (int64_t)0, (int)c->u12_async);
+          launch_k(c->pdl, k_u12g<16, kSplitBf16x2>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2], s[3], (int64_t)0, (int)c->u12_async, PW);
         else if (pg)
           launch_k(c->pdl, k_u12g<16, kSplitTf32>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2],
-                                                                                     xsplit ? nullptr : s[3], (int64_t)0, (int)c->u12_async);
+                                                                                     xsplit ? nullptr : s[3], (int64_t)0, (int)c->u12_async, PW);
         else if (bf16)
           launch_k(c->pdl, k_u12<16, 1, true>, g, CfgN::THREADS, CfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2], s[3]);
         else
@@ -1417,13 +1569,13 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
             const unsigned gw = (unsigned)((n - knext + 63) / 64);
             if (x3 && c->u12_wide)
               launch_k(c->pdl, k_u12g<64, kSplitBf16x2>, gw, GCfgW::THREADS, GCfgW::smem(), c->stream, A, lda, K0, knext, n,
-                       dinv, bh, b16(s[3]), (int64_t)0, (int)c->u12_async);
+                       dinv, bh, b16(s[3]), (int64_t)0, (int)c->u12_async, PW);
             else if (x3)
               launch_k(c->pdl, k_u12g<32, kSplitBf16x2>, g, GCfgR::THREADS, GCfgR::smem(), c->stream, A, lda, K0, knext, n, dinv, bh,
-                                                                                          b16(s[3]), (int64_t)0, (int)c->u12_async);
+                                                                                          b16(s[3]), (int64_t)0, (int)c->u12_async, PW);
             else if (pg)
               launch_k(c->pdl, k_u12g<32, kSplitTf32>, g, GCfgR::THREADS, GCfgR::smem(), c->stream, 
-                  A, lda, K0, knext, n, dinv, bh, xsplit ? nullptr : s[3] + (knext - kend) * PW, (int64_t)0, (int)c->u12_async);
+                  A, lda, K0, knext, n, dinv, bh, xsplit ? nullptr : s[3] + (knext - kend) * PW, (int64_t)0, (int)c->u12_async, PW);
             else if (bf16)
               launch_k(c->pdl, k_u12<32, 2, true>, g, CfgR::THREADS, CfgR::smem(), c->stream, A, lda, K0, knext, n, dinv, bh, nullptr);
             else

@@ -701,6 +701,178 @@ k_tc_gemm_multi(const __grid_constant__ CUtensorMap tmAh, const __grid_constant_
 }
 
 
+// ---------------------------------------------------------------------------
+// The BF16-pair update for large C: 128 x 256 tiles (N = 256 MMAs read a third
+// less shared memory per multiplication than N = 128), one CTA an SM with a
+// ring of four 32-deep K blocks (192 KB) and two accumulators, so that the
+// reduction of one tile into C runs beside the MMAs of the next. A CTA takes
+// tiles_per_cta tiles and leaves: the panel kernels of the factorisation, of
+// higher priority, get the SMs that become free.
+//   warp 0 / lane 0   TMA producer;
+//   warp 1 / lane 0   6 MMAs a K block (hi lo, lo hi, hi hi for two 16-deep steps);
+//   warps 2 .. 5      red.global.add of -D from the registers (lane = row).
+// Alone, C of 11,520 x 11,520 with 256 columns: 265 us, the MMAs without the
+// reductions 122 us (1.67 PFLOP/s), the reductions without the MMAs 225 us (4.7
+// TB/s of C read and written; loads and stores in the same tiles 3.3, a plain copy
+// of it 6.6): hence 512 columns a pass (lu_static_groups). Tiles of a CTA lie below
+// one another; neighbouring CTAs' tiles taken alternately cost 2 % at 36,600.
+namespace x3 {
+constexpr int WN = 256, KB = 32, STAGES = 4, THREADS = 192;
+constexpr int A_BYTES = BM * KB * 2, B_BYTES = WN * KB * 2, STAGE = 2 * A_BYTES + 2 * B_BYTES;
+constexpr int SMEM = STAGES * STAGE + 1024 + 256;
+constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(WN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(IDESC), "r"(accum), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+}  // namespace x3
+
+__global__ void __launch_bounds__(x3::THREADS, 1)
+k_tc_x3(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
+        const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, int m, int n, int K,
+        int tiles_per_cta, int* __restrict__ status, float* __restrict__ Cp, int64_t ldc) {
+  using namespace x3;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);
+  uint64_t* empty = full + STAGES;
+  uint64_t* accf = empty + STAGES;
+  uint64_t* acce = accf + 2;
+  uint64_t* drain = acce + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nk = (K + KB - 1) / KB;
+  const int mtiles = (m + BM - 1) / BM, ntiles = mtiles * ((n + WN - 1) / WN);
+  const int t0 = blockIdx.x * tiles_per_cta;
+  const int t1 = min(ntiles, t0 + tiles_per_cta);
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&accf[b], 1); mbar_init(&acce[b], 4); }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(2 * WN)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  griddep_wait();   // the operands and C come from the stream's earlier kernels
+
+  if (warp == 0) {
+    if (lane == 0) {   // producer
+      int it = 0, issued = 0;
+      for (int t = t0; t < t1 && !*(volatile int*)abort_flag; ++t) {
+        const int m0 = (t % mtiles) * BM, n0 = (t / mtiles) * WN;
+        for (int kb = 0; kb < nk; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1)) { *(volatile int*)abort_flag = 1; break; }
+          if (*(volatile int*)abort_flag) break;
+          mbar_expect_tx(&full[s], STAGE);
+          uint8_t* base = smem + s * STAGE;
+          tma_load_2d(base, &tmAh, kb * KB, m0, &full[s]);
+          tma_load_2d(base + A_BYTES, &tmAl, kb * KB, m0, &full[s]);
+          tma_load_2d(base + 2 * A_BYTES, &tmBh, kb * KB, n0, &full[s]);
+          tma_load_2d(base + 2 * A_BYTES + B_BYTES, &tmBl, kb * KB, n0, &full[s]);
+          issued = it + 1;
+        }
+      }
+      if (*(volatile int*)abort_flag)   // drain the copies this CTA issued before leaving
+        for (int q = (issued > STAGES ? issued - STAGES : 0); q < issued; ++q)
+          mbar_wait(&full[q % STAGES], (q / STAGES) & 1);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {   // MMA issuer
+      int it = 0, u = 0;
+      for (int t = t0; t < t1 && !*(volatile int*)abort_flag; ++t, ++u) {
+        const int b = u & 1;
+        if (u >= 2 && !mbar_wait(&acce[b], ((u >> 1) - 1) & 1)) { *(volatile int*)abort_flag = 1; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t acc = tmem + (uint32_t)(b * WN);
+        bool ok = true;
+        for (int kb = 0; kb < nk; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&full[s], (it / STAGES) & 1)) { ok = false; *(volatile int*)abort_flag = 1; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t base = smem_u32(smem + s * STAGE);
+          const uint64_t dAh = sdesc(base), dAl = sdesc(base + A_BYTES);
+          const uint64_t dBh = sdesc(base + 2 * A_BYTES), dBl = sdesc(base + 2 * A_BYTES + B_BYTES);
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {   // 16 bf16 = 32 bytes along K per MMA
+            const uint64_t off = (uint64_t)((kk * 32) >> 4);
+            umma(acc, dAh + off, dBl + off, (kb | kk) != 0 ? 1u : 0u);
+            umma(acc, dAl + off, dBh + off, 1u);
+            umma(acc, dAh + off, dBh + off, 1u);
+          }
+          umma_commit(&empty[s]);
+        }
+        if (!ok) break;
+        umma_commit(&accf[b]);
+      }
+      if (*(volatile int*)abort_flag && it > 0) {   // MMAs still in flight must finish before TMEM is freed
+        umma_commit(drain);
+        mbar_wait(drain, 0);
+      }
+    }
+  } else {   // epilogue
+    const int q = warp & 3;   // TMEM lanes 32 q .. 32 q + 31 = tile rows
+    int u = 0;
+    for (int t = t0; t < t1; ++t, ++u) {
+      const int b = u & 1;
+      const int64_t row = (int64_t)(t % mtiles) * BM + q * 32 + lane;
+      const int n0 = (t / mtiles) * WN;
+      // warp-uniform: tcgen05.ld is a .sync.aligned warp instruction
+      if (!__all_sync(0xffffffffu, mbar_wait(&accf[b], (u >> 1) & 1))) {
+        if (lane == 0) *(volatile int*)abort_flag = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float* cp = Cp + (int64_t)n0 * ldc + row;
+#pragma unroll 1
+      for (int cc = 0; cc < WN; cc += 16) {
+        uint32_t r[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * WN + cc)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (row < m) {
+          const int nc = n - (n0 + cc);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (j < nc) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(cp), "f"(-__uint_as_float(r[j])) : "memory");
+            cp += ldc;
+          }
+        } else {
+          cp += 16 * ldc;
+        }
+      }
+      // every TMEM read of this accumulator has completed: release it to the MMA warp
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acce[b]);
+    }
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0 && *(volatile int*)abort_flag) atomicOr(status, (int)DEV_TIMEOUT);
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * WN) : "memory");
+}
+
 // L21 panel (m x K, column-major, lda) -> K-major copies Ah, Al (m x ldk, row-major).
 __global__ void k_split_A(const float* __restrict__ A, int64_t lda, int m, int K, int ldk,
                           float* __restrict__ Ah, float* __restrict__ Al) {
@@ -932,18 +1104,40 @@ bool tc_gemm_sub_bf16x3(fp_ctx* c, const void* Ah, const void* Al, const void* B
   static SmemAttr a2, a6;
   if (a2.ensure(tc::k_tc_gemm_sub<2, true, true, true>, kTcSmemMax) != cudaSuccess) return false;
   if (a6.ensure(tc::k_tc_gemm_sub<6, true, true, true>, kTcSmemMax) != cudaSuccess) return false;
-  auto map16 = [&](CUtensorMap* tm, const void* base, int64_t rows) {
+  auto map16 = [&](CUtensorMap* tm, const void* base, int64_t rows, int box_rows) {
     cuuint64_t dims[2] = {(cuuint64_t)kk, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)ldk * 2};
-    cuuint32_t box[2] = {32u, (cuuint32_t)tc::BM};
+    cuuint32_t box[2] = {32u, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
     return tc::encode_fn()(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   CUtensorMap mAh, mAl, mBh, mBl, mC;
-  if (!map16(&mAh, Ah, m) || !map16(&mAl, Al, m) || !map16(&mBh, Bh, nn) || !map16(&mBl, Bl, nn) ||
-      !tc::make_map_c(&mC, C, m, nn, ldc, 32))
+  // two waves of the wide tiles or more, several panels' columns: k_tc_x3 (its
+  // single CTA an SM needs the tiles to overlap; with one panel's 128 columns the
+  // reductions into C bound both). 36,600 unknowns, all the updates, 512 columns:
+  // factorisation 161 -> 113 ms against 128 x 128 tiles with 256 columns, of which
+  // 145 with 256 columns. Eight tiles a CTA at most (113 ms; 114 with four, 117
+  // with two), four CTAs an SM or more, for the panel kernels that wait for SMs.
+  const int64_t wide = ((m + tc::BM - 1) / tc::BM) * ((nn + tc::x3::WN - 1) / tc::x3::WN);
+  if (kk > kStaticPanel && wide >= 2 * num_sms()) {
+    static SmemAttr aw;
+    if (aw.ensure(tc::k_tc_x3, tc::x3::SMEM) != cudaSuccess) return false;
+    if (!map16(&mAh, Ah, m, tc::BM) || !map16(&mAl, Al, m, tc::BM) || !map16(&mBh, Bh, nn, tc::x3::WN) ||
+        !map16(&mBl, Bl, nn, tc::x3::WN))
+      return false;
+    const int tpc = (int)std::max<int64_t>(1, std::min<int64_t>(8, wide / (4 * num_sms())));
+    const int ev = kt_begin(c);
+    TraceScope tr(c, TR_GEMM_TC);
+    launch_k(c->pdl, tc::k_tc_x3, dim3((unsigned)((wide + tpc - 1) / tpc)), dim3(tc::x3::THREADS), (size_t)tc::x3::SMEM,
+             c->stream, mAh, mAl, mBh, mBl, (int)m, (int)nn, kk, tpc, c->d_status, C, ldc);
+    kt_end(c, ev, 2.0 * (double)m * (double)nn * (double)kk, (double)m * (double)nn);
+    ++c->nlaunch;
+    return cudaGetLastError() == cudaSuccess;
+  }
+  if (!map16(&mAh, Ah, m, tc::BM) || !map16(&mAl, Al, m, tc::BM) || !map16(&mBh, Bh, nn, tc::BM) ||
+      !map16(&mBl, Bl, nn, tc::BM) || !tc::make_map_c(&mC, C, m, nn, ldc, 32))
     return false;
   dim3 grid((unsigned)((m + tc::BM - 1) / tc::BM), (unsigned)((nn + tc::BN - 1) / tc::BN));
   const int ev = kt_begin(c);
