@@ -27,8 +27,8 @@
 //               the split operands, with no separate split pass.
 // Look-ahead on two streams (lu_factor_static): the panel stream runs K1, K6,
 // then (after the previous panel's trailing update) K2 and K3 on the next
-// panel's columns; the second stream runs K2 and K5 on the columns beyond. Large systems
-// in the BF16-pair form go by groups of panels instead (lu_static_groups).
+// panel's columns; the second stream runs K2 and K5 on the columns beyond. The
+// BF16-pair form goes by groups of panels instead (lu_static_groups).
 // The panel width equals the triangular solves' 128-row blocks.
 #include <cuda_bf16.h>
 
@@ -181,7 +181,8 @@ __device__ __forceinline__ void store_block(float* __restrict__ g, int64_t ld, i
 // U on and above the diagonal); the inverses of its IB x IB diagonal blocks
 // of L and U go to dinv. Rows and columns past n are padded with the identity.
 // 256 threads and 85 KB of shared memory, so that the CTA fits on an SM
-// beside two CTAs of the tensor-core update of the second stream.
+// beside two CTAs of the tensor-core update of the second stream. Used where the
+// full inv(L) is wanted too (FP_TUNE_PDIAG_LINV), else k_pdiag_reg below.
 //
 // Per inner block kb (columns k0 .. k0 + 31):
 //   (a) warp 0 eliminates the IB x IB diagonal block (eliminate);
@@ -484,6 +485,210 @@ k_pdiag(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, float* __restr
   if (linvt != nullptr && nb == PW) full_linv(As, LT, Dl, linvt, tid);
 }
 
+// K1 without the full inverse: 16 warps own 8 columns each, lane i rows 4 i ..
+// 4 i + 3, all in registers. A column's step needs its pivot (one shuffle), the
+// reciprocal and the multipliers; they go to the other warps through Ls and a
+// barrier a column, and each warp applies them to its own columns with the
+// pivot row's entries from a shuffle. The warp that owns the next columns follows
+// four columns at a time, the others eight. A serial chain of 128 steps bounds it:
+// about 75 cycles a column within a warp, 500 from one warp's last column to the
+// next one's first (1,000 while most warps have work). The 32 x 32 inverses by
+// blocks of 8 (1.4 us; as one substitution of 32 steps 5 to 7). A block alone 25.2
+// -> 21.0 us, 18 of them in the kernel (27.3 -> 30.5 with a wait for each column
+// and those substitutions).
+constexpr int kPdiagThreads = 512;
+constexpr int XB = IB + 4;   // row pitch of the 32 x 32 blocks
+constexpr size_t pdiag_reg_smem() { return ((size_t)PW * PW + (size_t)NIB * 3 * IB * XB) * sizeof(float); }
+__device__ __forceinline__ void wait_column(uint64_t* bar, int* status) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
+  bool done = false;
+  for (int i = 0; i < (1 << 16) && !done; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(a)
+        : "memory");
+    done = ok != 0;
+  }
+  if (!done) atomicOr(status, (int)DEV_TIMEOUT);
+  __syncwarp();
+}
+// One warp: the inverse of a lower triangular 32 x 32 block M (D itself, unit
+// diagonal, or the transpose of the upper triangle D) into X: the 8 x 8 diagonal
+// blocks by substitution, a lane a column of one, then twice the block below the
+// diagonal of a pair, X21 = -X22 (M21 X11).
+template <bool Upper>
+__device__ __forceinline__ void invert_block(const float (*D)[XB], float (*X)[XB], float* __restrict__ out, int lane) {
+  const auto M = [&](int r, int c) { return Upper ? D[c][r] : D[r][c]; };
+#pragma unroll 4
+  for (int i = 0; i < IB; ++i) X[i][lane] = 0.f;
+  __syncwarp();
+  {
+    const int o = lane & ~7, c = lane & 7;
+    float x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float t = i == c ? 1.f : 0.f;
+#pragma unroll
+      for (int q = 0; q < i; ++q) t = fmaf(-M(o + i, o + q), x[q], t);
+      x[i] = Upper ? t * rcp_fast(M(o + i, o + i)) : t;
+      X[o + i][o + c] = x[i];
+    }
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int h = 8; h < IB; h *= 2) {
+    // lanes over the 16 / h pairs, their h rows and h * h / 32 * (16 / h) = h / 2 columns a lane
+    const int per = 2 * h, o = (lane / per) * per, r = (lane % per) >> 1, c0 = (lane & 1) * (h / 2);
+    const int w = h / 2;   // 4 or 8 columns a lane
+    float t[8] = {};
+    for (int q = 0; q < h; ++q) {
+      const float m = M(o + h + r, o + q);
+#pragma unroll
+      for (int e = 0; e < 8; e += 4)
+        if (e < w) {
+          const float4 v = *reinterpret_cast<const float4*>(&X[o + q][o + c0 + e]);
+          t[e] = fmaf(m, v.x, t[e]); t[e + 1] = fmaf(m, v.y, t[e + 1]);
+          t[e + 2] = fmaf(m, v.z, t[e + 2]); t[e + 3] = fmaf(m, v.w, t[e + 3]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e += 4)
+      if (e < w) *reinterpret_cast<float4*>(&X[o + h + r][o + c0 + e]) = make_float4(t[e], t[e + 1], t[e + 2], t[e + 3]);
+    __syncwarp();
+    float y[8] = {};
+    for (int q = 0; q < h; ++q) {
+      const float m = X[o + h + r][o + h + q];
+#pragma unroll
+      for (int e = 0; e < 8; e += 4)
+        if (e < w) {
+          const float4 v = *reinterpret_cast<const float4*>(&X[o + h + q][o + c0 + e]);
+          y[e] = fmaf(m, v.x, y[e]); y[e + 1] = fmaf(m, v.y, y[e + 1]);
+          y[e + 2] = fmaf(m, v.z, y[e + 2]); y[e + 3] = fmaf(m, v.w, y[e + 3]);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 8; e += 4)
+      if (e < w) *reinterpret_cast<float4*>(&X[o + h + r][o + c0 + e]) = make_float4(-y[e], -y[e + 1], -y[e + 2], -y[e + 3]);
+    __syncwarp();
+  }
+#pragma unroll 8
+  for (int i = 0; i < IB; ++i) out[i * IB + lane] = Upper ? X[lane][i] : X[i][lane];
+}
+// the multipliers of column j = 8 b + jj (in l) applied to the columns [first, 8)
+// of a warp; jl, js: the lane and slot of row j
+__device__ __forceinline__ void apply_column(float (&a)[8][4], const float4 l, int jl, int js, int first) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    if (c < first) continue;
+    const float u = __shfl_sync(FULL, a[c][js], jl);
+    a[c][0] = fmaf(-l.x, u, a[c][0]);
+    a[c][1] = fmaf(-l.y, u, a[c][1]);
+    a[c][2] = fmaf(-l.z, u, a[c][2]);
+    a[c][3] = fmaf(-l.w, u, a[c][3]);
+  }
+}
+__global__ void __launch_bounds__(kPdiagThreads, 1)
+k_pdiag_reg(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, float* __restrict__ dinv,
+            float* __restrict__ cert, int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ uint64_t step[PW];
+  float (*Ls)[PW] = reinterpret_cast<float (*)[PW]>(smem);   // the multipliers by column, 0 on and above the diagonal
+  // per diagonal block of 32: the block, its inverses' work space
+  float (*Ds)[XB] = reinterpret_cast<float (*)[XB]>(smem + (size_t)PW * PW * sizeof(float));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < PW) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((uint32_t)__cvta_generic_to_shared(&step[tid])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  griddep_wait();
+  const int nb = (int)imin64(PW, n - k), r0 = 4 * lane, own = 8 * warp;
+  float* const g = A + (k + own) * lda + k + r0;
+  float a[8][4];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {   // past the end: the identity
+    if (own + c < nb && r0 + 4 <= nb) {
+      const float4 v = *reinterpret_cast<const float4*>(g + c * lda);
+      a[c][0] = v.x; a[c][1] = v.y; a[c][2] = v.z; a[c][3] = v.w;
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        a[c][r] = own + c < nb && r0 + r < nb ? g[c * lda + r] : (r0 + r == own + c ? 1.f : 0.f);
+    }
+  }
+#pragma unroll 1
+  for (int b = 0; b < warp; ++b) {
+    if (b < warp - 1) wait_column(&step[8 * b + 7], status);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      if (b == warp - 1) wait_column(&step[8 * b + 4 * half + 3], status);
+      float4 l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) l[q] = *reinterpret_cast<const float4*>(&Ls[8 * b + 4 * half + q][r0]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) apply_column(a, l[q], 2 * b + half, q, 0);
+    }
+  }
+  bool bad = false;
+  float lmax = 0.f;
+#pragma unroll
+  for (int jj = 0; jj < 8; ++jj) {
+    const int js = jj & 3, jl = 2 * warp + (jj >> 2);
+    const float p = __shfl_sync(FULL, a[jj][js], jl);
+    bad |= !(fabsf(p) > 0.f && fabsf(p) <= FLT_MAX);
+    const float rp = rcp_fast(p);
+    float l[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const bool below = lane > jl || (lane == jl && r > js);
+      l[r] = below ? a[jj][r] * rp : 0.f;
+      if (below) a[jj][r] = l[r];
+      lmax = fmaxf(lmax, fabsf(l[r]));
+    }
+    const float4 lv = make_float4(l[0], l[1], l[2], l[3]);
+    *reinterpret_cast<float4*>(&Ls[own + jj][r0]) = lv;
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"((uint32_t)__cvta_generic_to_shared(&step[own + jj]))
+                   : "memory");
+    apply_column(a, lv, jl, js, jj + 1);
+  }
+  if (bad && lane == 0) atomicOr(status, (int)DEV_ZERO_PIVOT);
+  griddep_launch();
+  // the factors back, and the diagonal block (of four warps) for the inverses
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    if (own + c >= nb) break;
+    if (r0 + 4 <= nb) {
+      *reinterpret_cast<float4*>(g + c * lda) = make_float4(a[c][0], a[c][1], a[c][2], a[c][3]);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r0 + r < nb) g[c * lda + r] = a[c][r];
+    }
+  }
+  const int blk = warp >> 2;
+  float (*D)[XB] = Ds + blk * 3 * IB;
+  if (r0 / IB == blk)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      float* const d = &D[r0 % IB + r][own % IB];
+      *reinterpret_cast<float4*>(d) = make_float4(a[0][r], a[1][r], a[2][r], a[3][r]);
+      *reinterpret_cast<float4*>(d + 4) = make_float4(a[4][r], a[5][r], a[6][r], a[7][r]);
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(FULL, lmax, o));
+  if (lane == 0) atomic_max_pos(cert, lmax);
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + blk) : "memory");
+  if ((warp & 3) == 0) invert_block<true>(D, D + IB, dinv + dinv_off(blk, 1), lane);
+  else if ((warp & 3) == 1) invert_block<false>(D, D + 2 * IB, dinv + dinv_off(blk, 0), lane);
+}
+
 // The split of four consecutive K values of a K-major operand at o (element
 // offset), by split mode SM: kSplitTf32 TF32 hi / lo (unsplit FP32 when lo is
 // null), kSplitBf16 BF16 (the BF16 form; no lo), kSplitBf16x2 BF16 hi / lo
@@ -636,21 +841,19 @@ struct U12Cfg {
   }
 };
 
-template <int CW, int RT, bool BF16>
-__global__ void __launch_bounds__(U12Cfg<CW, RT>::THREADS)
-k_u12(float* __restrict__ A, int64_t lda, int64_t k, int64_t c0, int64_t c1, const float* __restrict__ dinv,
-      float* __restrict__ Bh, float* __restrict__ Bl) {
-  griddep_wait();
+template <int CW, int RT, int SM>
+__device__ __forceinline__ void u12(unsigned char* smem, int block, float* __restrict__ A, int64_t lda, int64_t k, int64_t c0,
+                                    int64_t c1, const float* __restrict__ dinv, float* __restrict__ Bh,
+                                    float* __restrict__ Bl, int ldo) {
   typedef U12Cfg<CW, RT> Cfg;
   constexpr int T = Cfg::THREADS, ZP = Cfg::ZP, LP = Cfg::LP;
-  extern __shared__ __align__(16) unsigned char smem[];
   float (*Z)[ZP] = reinterpret_cast<float (*)[ZP]>(smem);                                    // PW x CW
   // Lb[r - IB][s] = L(r, s) for r >= 32, s < 96 (entries right of the diagonal blocks are not read)
   float (*Lb)[LP] = reinterpret_cast<float (*)[LP]>(smem + (size_t)PW * ZP * sizeof(float));
   float (*Lt)[UP] = reinterpret_cast<float (*)[UP]>(reinterpret_cast<unsigned char*>(Lb) +
                                                      (size_t)(PW - IB) * LP * sizeof(float));   // inv(L_tt), 4 x 32 rows
   const int tid = threadIdx.x;
-  const int64_t col0 = c0 + (int64_t)blockIdx.x * CW;
+  const int64_t col0 = c0 + (int64_t)block * CW;
   const int cols = (int)imin64(CW, c1 - col0);
   {   // all loads in flight before the first store
     const auto zero = [](int, int) { return 0.f; };
@@ -711,21 +914,17 @@ k_u12(float* __restrict__ A, int64_t lda, int64_t k, int64_t c0, int64_t c1, con
   for (int e = tid; e < cols * R4; e += T) {   // the split, K-major: column j - c0 holds its PW values
     const int c = e / R4, r = (e % R4) * 4;
     const float v[4] = {Z[r][c], Z[r + 1][c], Z[r + 2][c], Z[r + 3][c]};
-    const int64_t o = (col0 - c0 + c) * (int64_t)PW + r;
-    if (BF16) {
-      __nv_bfloat162* d = reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(Bh) + o);
-      d[0] = __floats2bfloat162_rn(v[0], v[1]);
-      d[1] = __floats2bfloat162_rn(v[2], v[3]);
-    } else if (Bl) {
-      float h[4], lo[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) { h[i] = tf32_rna(v[i]); lo[i] = v[i] - h[i]; }
-      *reinterpret_cast<float4*>(&Bh[o]) = make_float4(h[0], h[1], h[2], h[3]);
-      *reinterpret_cast<float4*>(&Bl[o]) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-    } else {   // unsplit: the update splits in shared memory
-      *reinterpret_cast<float4*>(&Bh[o]) = make_float4(v[0], v[1], v[2], v[3]);
-    }
+    put_split<SM>(Bh, Bl, (col0 - c0 + c) * (int64_t)ldo + r, v);
   }
+}
+
+template <int CW, int RT, int SM>
+__global__ void __launch_bounds__(U12Cfg<CW, RT>::THREADS)
+k_u12(float* __restrict__ A, int64_t lda, int64_t k, int64_t c0, int64_t c1, const float* __restrict__ dinv,
+      float* __restrict__ Bh, float* __restrict__ Bl, int ldo) {
+  griddep_wait();
+  extern __shared__ __align__(16) unsigned char smem[];
+  u12<CW, RT, SM>(smem, blockIdx.x, A, lda, k, c0, c1, dinv, Bh, Bl, ldo);
 }
 
 // ---------------------------------------------------------------------------
@@ -770,17 +969,15 @@ constexpr size_t l21a_smem() {
   return ((size_t)PW * XTP + (size_t)(PW - IB) * UTP + (size_t)NIB * IB * UP) * sizeof(float);
 }
 template <int SM>
-__global__ void __launch_bounds__(L21_THREADS)
-k_l21a(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int64_t rbeg,
-       const float* __restrict__ dinv, float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert, int ldo) {
-  griddep_wait();
-  extern __shared__ __align__(16) unsigned char smem[];
+__device__ __forceinline__ void l21a(unsigned char* smem, int block, float* __restrict__ A, int64_t lda, int64_t n, int64_t k,
+                                     int64_t r0, int64_t rbeg, const float* __restrict__ dinv, float* __restrict__ Ah,
+                                     float* __restrict__ Al, float* __restrict__ cert, int ldo) {
   float (*XT)[XTP] = reinterpret_cast<float (*)[XTP]>(smem);
   float (*UbT)[UTP] = reinterpret_cast<float (*)[UTP]>(smem + (size_t)PW * XTP * sizeof(float));
   float (*Ut)[UP] = reinterpret_cast<float (*)[UP]>(reinterpret_cast<unsigned char*>(UbT) +
                                                      (size_t)(PW - IB) * UTP * sizeof(float));
   const int tid = threadIdx.x;
-  const int64_t row0 = rbeg + (int64_t)blockIdx.x * L21_ROWS;
+  const int64_t row0 = rbeg + (int64_t)block * L21_ROWS;
   const int rows = (int)imin64(L21_ROWS, n - row0);
 #pragma unroll
   for (int u = 0; u < PW * (L21_ROWS / 4) / L21_THREADS; ++u) {   // XT: 128 columns x 8 chunks of 4 rows
@@ -871,6 +1068,32 @@ k_l21a(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(FULL, lmax, o));
   if ((tid & 31) == 0) atomic_max_pos(cert, lmax);
+}
+
+template <int SM>
+__global__ void __launch_bounds__(L21_THREADS)
+k_l21a(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, int64_t r0, int64_t rbeg,
+       const float* __restrict__ dinv, float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ cert, int ldo) {
+  griddep_wait();
+  extern __shared__ __align__(16) unsigned char smem[];
+  l21a<SM>(smem, blockIdx.x, A, lda, n, k, r0, rbeg, dinv, Ah, Al, cert, ldo);
+}
+
+// K6 on the rows [k1, k2) and K2 on the columns [k1, k2) in one launch, both by
+// block substitution: the chain of the group form waits for one kernel after K1,
+// 12,000 unknowns 7.0 -> 6.7 ms against K6 and then K2 as a product with inv(L).
+static_assert(U12Cfg<16, 1>::THREADS == L21_THREADS, "one block size");
+constexpr size_t next_smem() { return std::max(l21a_smem(), U12Cfg<16, 1>::smem()); }
+template <int SM>
+__global__ void __launch_bounds__(L21_THREADS)
+k_next(float* __restrict__ A, int64_t lda, int64_t k, int64_t k1, int64_t k2, int64_t r0, const float* __restrict__ dinv,
+       float* __restrict__ Ah, float* __restrict__ Al, float* __restrict__ Bh, float* __restrict__ Bl, float* __restrict__ cert,
+       int ldo) {
+  griddep_wait();
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int nl = (int)((k2 - k1 + L21_ROWS - 1) / L21_ROWS);
+  if ((int)blockIdx.x < nl) l21a<SM>(smem, blockIdx.x, A, lda, k2, k, r0, k1, dinv, Ah, Al, cert, ldo);
+  else u12<16, 1, SM>(smem, blockIdx.x - nl, A, lda, k, k1, k2, dinv, Bh, Bl, ldo);
 }
 
 // K1b: 2 NIB CTAs. CTA b < NIB forms block column j = b of inv(L), CTA
@@ -1154,11 +1377,11 @@ __global__ void k_iota(int32_t* __restrict__ ipiv, int64_t n) {
 // panel, the next group's columns and rows come first, and the next group's panels
 // run beside the rest of the update. With panel p of the group at columns
 // [k, k1), k2 the end of the next one, F the group's end and H the next group's:
-//   stream   the chain of diagonal blocks: K1, K6 on rows [k1, k2), K2 on columns
-//            [k1, k2), update of the tile [k1, k2) x [k1, k2)
-//   stream3  inv(L); K6 on the rows from k2 on, then their update in the next
-//            panel's columns (after the last panel: in [F, H))
-//   stream4  K2 on the columns from k2 on, then their update in the next panel's
+//   stream   the chain of diagonal blocks: K1, K6 and K2 on the next panel's rows and
+//            columns (k_next), update of the tile [k1, k2) x [k1, k2)
+//   stream3  K6 on the rows from k2 on, then their update in the next panel's columns
+//            (after the last panel: in [F, H))
+//   stream4  inv(L), K2 on the columns from k2 on, then their update in the next panel's
 //            rows (after the last panel: also in the rows up to H)
 //   stream2  after the last panel: [H, n) x [H, n)
 // The split operands hold the group's 128 G K values a row; rows and columns count
@@ -1172,7 +1395,8 @@ static int lu_static_groups(fp_ctx* c, float* A, int64_t n, int64_t lda, float* 
   float* const dinv_base = reinterpret_cast<float*>(c->d_minv);
   const auto at = [&](int64_t r, int64_t col) { return A + col * lda + r; };
   const auto wait = [&](cudaStream_t s, cudaEvent_t e) { return cudaStreamWaitEvent(s, e, 0); };
-  const cudaStream_t s1 = c->stream, s2 = c->stream2, s3 = c->stream3, s4 = c->stream4;
+  const cudaStream_t s1 = c->stream, s2 = c->stream2, s3 = c->stream3;
+  const cudaStream_t s4 = n > 2 * LD ? c->stream4 : c->stream2;   // two groups: nothing is left to the second stream
   for (cudaEvent_t e : {c->ev_rest, c->ev_tcr, c->ev_top}) FP_CUDA_TRY(c->err, cudaEventRecord(e, s1));
   for (int64_t i = 0; i * PW < n; ++i) {
     const int p = (int)(i % G), kk = (p + 1) * PW, set = (int)((i / G) & 1);
@@ -1194,72 +1418,67 @@ static int lu_static_groups(fp_ctx* c, float* A, int64_t n, int64_t lda, float* 
         if (int rc = gemm_sub_simt_f32(c, at(r0, q), at(q, q0), at(r0, q0), lda, r1 - r0, q1 - q0, PW)) return rc;
       return FP_OK;
     };
-    const auto l21 = [&](int64_t r0, int64_t r1) -> int {
-      if (r0 >= r1) return FP_OK;
-      TraceScope tr(c, TR_L21);
-      launch_k(c->pdl, k_l21a<kSplitBf16x2>, (unsigned)((r1 - r0 + L21_ROWS - 1) / L21_ROWS), L21_THREADS, l21a_smem(),
-               c->stream, A, lda, r1, k, E, r0, dinv, reinterpret_cast<float*>(op[0] + p * PW),
-               reinterpret_cast<float*>(op[1] + p * PW), cert, LD);
-      ++c->nlaunch;
-      FP_CUDA_TRY(c->err, cudaGetLastError());
-      return FP_OK;
-    };
-    const auto u12 = [&](int64_t q0, int64_t q1, bool narrow) -> int {
-      if (q0 >= q1) return FP_OK;
-      TraceScope tr(c, narrow ? TR_U12 : TR_STRIP);
-      float* const bh = reinterpret_cast<float*>(op[2] + (q0 - E) * LD + p * PW);
-      float* const bl = reinterpret_cast<float*>(op[3] + (q0 - E) * LD + p * PW);
-      const auto go = [&](auto kernel, int cw, int threads, size_t smem) {
-        launch_k(c->pdl, kernel, (unsigned)((q1 - q0 + cw - 1) / cw), threads, smem, c->stream, A, lda, k, q0, q1, dinv, bh, bl,
-                 (int64_t)0, (int)c->u12_async, LD);
-      };
-      if (narrow) go(k_u12g<16, kSplitBf16x2>, 16, U12gCfg<16>::THREADS, U12gCfg<16>::smem());
-      else if (c->u12_wide) go(k_u12g<64, kSplitBf16x2>, 64, U12gCfg<64>::THREADS, U12gCfg<64>::smem());
-      else go(k_u12g<32, kSplitBf16x2>, 32, U12gCfg<32>::THREADS, U12gCfg<32>::smem());
-      ++c->nlaunch;
-      FP_CUDA_TRY(c->err, cudaGetLastError());
-      return FP_OK;
-    };
+    const auto opf = [&](int q, int64_t o) { return reinterpret_cast<float*>(op[q] + o); };
     // the chain. The slot of the inverses is free: what panel i - 2 left to the
     // other streams came before the updates that panel i - 1 waited for
     {
       TraceScope tr(c, TR_DIAG);
-      launch_k(c->pdl, k_pdiag, 1, kDiagThreads, pdiag_smem(false), s1, A, lda, n, k, dinv, cert, c->d_status, (float*)nullptr);
+      launch_k(c->pdl, k_pdiag_reg, 1, kPdiagThreads, pdiag_reg_smem(), s1, A, lda, n, k, dinv, cert, c->d_status);
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
     }
     if (k1 == n) break;
     FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_diag, s1));
+    FP_CUDA_TRY(c->err, wait(s1, c->ev_tcr));   // this panel's rows from k1 on
+    FP_CUDA_TRY(c->err, wait(s1, c->ev_top));   // its columns from k1 on
     {
-      OnStream on3(c, s3);
-      FP_CUDA_TRY(c->err, wait(s3, c->ev_diag));
-      TraceScope tr(c, TR_PINV);
-      launch_k(c->pdl, k_pinv, NIB, PI_THREADS, pinv_smem(), s3, A, lda, k, dinv);
+      TraceScope tr(c, TR_U12);
+      const unsigned g = (unsigned)((k2 - k1 + L21_ROWS - 1) / L21_ROWS + (k2 - k1 + 15) / 16);
+      launch_k(c->pdl, k_next<kSplitBf16x2>, g, L21_THREADS, next_smem(), s1, A, lda, k, k1, k2, E, dinv,
+               opf(0, p * PW), opf(1, p * PW), opf(2, (k1 - E) * LD + p * PW), opf(3, (k1 - E) * LD + p * PW),
+               cert, LD);
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
-      FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_pinv, s3));
     }
-    FP_CUDA_TRY(c->err, wait(s1, c->ev_tcr));   // this panel's rows from k1 on
-    if (int rc = l21(k1, k2)) return rc;
     FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_panel, s1));
-    FP_CUDA_TRY(c->err, wait(s1, c->ev_top));   // its columns from k1 on
-    FP_CUDA_TRY(c->err, wait(s1, c->ev_pinv));
-    if (int rc = u12(k1, k2, true)) return rc;
-    FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_u12n, s1));
     if (last) FP_CUDA_TRY(c->err, wait(s1, c->ev_rest));
     if (int rc = update(k1, k2, k1, k2)) return rc;
     if (k2 == n) continue;
     {
       OnStream on4(c, s4);   // U12 of the columns beyond
-      FP_CUDA_TRY(c->err, wait(s4, c->ev_pinv));
-      if (int rc = u12(k2, n, false)) return rc;
+      FP_CUDA_TRY(c->err, wait(s4, c->ev_diag));
+      {
+        TraceScope tr(c, TR_PINV);
+        launch_k(c->pdl, k_pinv, NIB, PI_THREADS, pinv_smem(), s4, A, lda, k, dinv);
+        ++c->nlaunch;
+        FP_CUDA_TRY(c->err, cudaGetLastError());
+      }
+      {
+        TraceScope tr(c, TR_STRIP);
+        const int64_t o = (k2 - E) * LD + p * PW;
+        const auto go = [&](auto kernel, int cw, int threads, size_t smem) {
+          launch_k(c->pdl, kernel, (unsigned)((n - k2 + cw - 1) / cw), threads, smem, s4, A, lda, k, k2, n, dinv, opf(2, o),
+                   opf(3, o), (int64_t)0, (int)c->u12_async, LD);
+        };
+        if (c->u12_wide) go(k_u12g<64, kSplitBf16x2>, 64, U12gCfg<64>::THREADS, U12gCfg<64>::smem());
+        else go(k_u12g<32, kSplitBf16x2>, 32, U12gCfg<32>::THREADS, U12gCfg<32>::smem());
+        ++c->nlaunch;
+        FP_CUDA_TRY(c->err, cudaGetLastError());
+      }
       FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_u12r, s4));
     }
     {
       OnStream on3(c, s3);   // the rows below
-      if (int rc = l21(k2, n)) return rc;
+      FP_CUDA_TRY(c->err, wait(s3, c->ev_diag));
+      {
+        TraceScope tr(c, TR_L21);
+        launch_k(c->pdl, k_l21a<kSplitBf16x2>, (unsigned)((n - k2 + L21_ROWS - 1) / L21_ROWS), L21_THREADS, l21a_smem(), s3, A,
+                 lda, n, k, E, k2, dinv, opf(0, p * PW), opf(1, p * PW), cert, LD);
+        ++c->nlaunch;
+        FP_CUDA_TRY(c->err, cudaGetLastError());
+      }
       FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_l21t, s3));
-      FP_CUDA_TRY(c->err, wait(s3, c->ev_u12n));
+      FP_CUDA_TRY(c->err, wait(s3, c->ev_panel));
       if (last) {
         FP_CUDA_TRY(c->err, wait(s3, c->ev_u12r));
         FP_CUDA_TRY(c->err, wait(s3, c->ev_rest));
@@ -1287,7 +1506,7 @@ static int lu_static_groups(fp_ctx* c, float* A, int64_t n, int64_t lda, float* 
     }
   }
   // the other streams' last work
-  for (cudaEvent_t e : {c->ev_rest, c->ev_tcr, c->ev_top, c->ev_pinv}) FP_CUDA_TRY(c->err, wait(s1, e));
+  for (cudaEvent_t e : {c->ev_rest, c->ev_tcr, c->ev_top}) FP_CUDA_TRY(c->err, wait(s1, e));
   return FP_OK;
 }
 
@@ -1301,7 +1520,7 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
   FP_CUDA_TRY(c->err, cudaMemsetAsync(cert, 0, sizeof(float), c->stream));
   typedef U12Cfg<16, 1> CfgN;   // the next panel's columns: many small CTAs
   typedef U12Cfg<32, 2> CfgR;   // the columns beyond
-  static SmemAttr attr_d, attr_l, attr_lx, attr_un, attr_ur, attr_lb, attr_unb, attr_urb, attr_la[3];
+  static SmemAttr attr_d, attr_dr, attr_l, attr_lx, attr_un, attr_ux, attr_ur, attr_lb, attr_unb, attr_urb, attr_la[3];
   FP_CUDA_TRY(c->err, attr_la[0].ensure(k_l21a<kSplitTf32>, (int)l21a_smem()));
   FP_CUDA_TRY(c->err, attr_la[1].ensure(k_l21a<kSplitBf16x2>, (int)l21a_smem()));
   FP_CUDA_TRY(c->err, attr_la[2].ensure(k_l21a<kSplitBf16>, (int)l21a_smem()));
@@ -1336,13 +1555,15 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
   // the FP32 form's update from BF16 pairs (needs the GEMM-form panel kernels)
   const bool x3 = !bf16 && pg && c->tc_x3 && c->use_tc;
   FP_CUDA_TRY(c->err, attr_d.ensure(k_pdiag, (int)pdiag_smem(true)));
+  FP_CUDA_TRY(c->err, attr_dr.ensure(k_pdiag_reg, (int)pdiag_reg_smem()));
   FP_CUDA_TRY(c->err, attr_l.ensure(k_l21<kSplitTf32>, (int)l21_smem()));
   FP_CUDA_TRY(c->err, attr_lx.ensure(k_l21<kSplitBf16x2>, (int)l21_smem()));
-  FP_CUDA_TRY(c->err, attr_un.ensure(k_u12<16, 1, false>, (int)CfgN::smem()));
-  FP_CUDA_TRY(c->err, attr_ur.ensure(k_u12<32, 2, false>, (int)CfgR::smem()));
+  FP_CUDA_TRY(c->err, attr_un.ensure(k_u12<16, 1, kSplitTf32>, (int)CfgN::smem()));
+  FP_CUDA_TRY(c->err, attr_ux.ensure(k_next<kSplitBf16x2>, (int)next_smem()));
+  FP_CUDA_TRY(c->err, attr_ur.ensure(k_u12<32, 2, kSplitTf32>, (int)CfgR::smem()));
   FP_CUDA_TRY(c->err, attr_lb.ensure(k_l21<kSplitBf16>, (int)l21_smem()));
-  FP_CUDA_TRY(c->err, attr_unb.ensure(k_u12<16, 1, true>, (int)CfgN::smem()));
-  FP_CUDA_TRY(c->err, attr_urb.ensure(k_u12<32, 2, true>, (int)CfgR::smem()));
+  FP_CUDA_TRY(c->err, attr_unb.ensure(k_u12<16, 1, kSplitBf16>, (int)CfgN::smem()));
+  FP_CUDA_TRY(c->err, attr_urb.ensure(k_u12<32, 2, kSplitBf16>, (int)CfgR::smem()));
   if (int rc = ensure_tc_scratch(c, 0, n)) return rc;
   if (int rc = ensure_tc_scratch(c, 1, n)) return rc;
   // the tensor-core update splits the operands in shared memory: L21 and U12
@@ -1356,11 +1577,12 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
   FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_rest, c->stream));
   if (c->rest_split) FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_top, c->stream));
   FP_CUDA_TRY(c->err, cudaStreamWaitEvent(c->stream2, c->ev_rest, 0));
-  // from 56 panels on by groups of four. Below, the chain of diagonal blocks bounds
-  // both forms (2,000 unknowns 0.97 ms, groups 0.98; 6,000 3.01, 3.06; 8,000 4.97,
-  // 4.40; 12,000 10.5, 8.1; 20,800 42.8, 24.6; 36,600 219, 113; groups of two: 4.58,
-  // 8.83, 30.9, 150; of three: 4.69, 8.63, 28.0, 131)
-  if (x3 && lside && !dl && c->lu_split && c->lu_overlap && !c->lu_fuse && !c->rest_split && c->l21_async && n >= 56 * PW)
+  // the BF16-pair form by groups of four panels (single panels in the chain below,
+  // both with k_pdiag_reg: 960 unknowns 0.46 ms, groups 0.42; 2,000 0.83, 0.76;
+  // 6,000 2.55, 2.34; with the earlier K1: 12,000 10.5, 8.1, now 6.7; 20,800 42.8,
+  // 23.5; 36,600 219, 113; groups of two: 8.8 at 12,000, 150 at 36,600; of three:
+  // 8.6, 131)
+  if (x3 && lside && !dl && c->lu_split && c->lu_overlap && !c->lu_fuse && !c->rest_split && c->l21_async)
     return lu_static_groups<4>(c, A, n, lda, cert);
   // C -= L21 U12 on the rows [kend, n) and columns [cb, ce): tensor cores from
   // the split operands, or the SIMT kernel on the factors in place
@@ -1402,8 +1624,10 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
     {
       TraceScope tr(c, TR_DIAG);
       float* const linvt = (dl && kend < n) ? dinv + kLinvtOff : nullptr;
-      launch_k(c->pdl, k_pdiag, 1, kDiagThreads, pdiag_smem(linvt != nullptr), c->stream, A, lda, n, K0, dinv, cert,
-               c->d_status, linvt);
+      if (linvt)
+        launch_k(c->pdl, k_pdiag, 1, kDiagThreads, pdiag_smem(true), c->stream, A, lda, n, K0, dinv, cert, c->d_status, linvt);
+      else
+        launch_k(c->pdl, k_pdiag_reg, 1, kPdiagThreads, pdiag_reg_smem(), c->stream, A, lda, n, K0, dinv, cert, c->d_status);
       ++c->nlaunch;
       FP_CUDA_TRY(c->err, cudaGetLastError());
     }
@@ -1525,10 +1749,10 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
           launch_k(c->pdl, k_u12g<16, kSplitTf32>, g, GCfgN::THREADS, GCfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2],
                                                                                      xsplit ? nullptr : s[3], (int64_t)0, (int)c->u12_async, PW);
         else if (bf16)
-          launch_k(c->pdl, k_u12<16, 1, true>, g, CfgN::THREADS, CfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2], s[3]);
+          launch_k(c->pdl, k_u12<16, 1, kSplitBf16>, g, CfgN::THREADS, CfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2], s[3], PW);
         else
-          launch_k(c->pdl, k_u12<16, 1, false>, g, CfgN::THREADS, CfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2],
-                                                                              xsplit ? nullptr : s[3]);
+          launch_k(c->pdl, k_u12<16, 1, kSplitTf32>, g, CfgN::THREADS, CfgN::smem(), c->stream, A, lda, K0, kend, knext, dinv, s[2],
+                   xsplit ? nullptr : s[3], PW);
         ++c->nlaunch;
         FP_CUDA_TRY(c->err, cudaGetLastError());
       }
@@ -1577,10 +1801,10 @@ int lu_factor_static(fp_ctx* c, float* A, int64_t n, int64_t lda, int32_t* ipiv,
               launch_k(c->pdl, k_u12g<32, kSplitTf32>, g, GCfgR::THREADS, GCfgR::smem(), c->stream, 
                   A, lda, K0, knext, n, dinv, bh, xsplit ? nullptr : s[3] + (knext - kend) * PW, (int64_t)0, (int)c->u12_async, PW);
             else if (bf16)
-              launch_k(c->pdl, k_u12<32, 2, true>, g, CfgR::THREADS, CfgR::smem(), c->stream, A, lda, K0, knext, n, dinv, bh, nullptr);
+              launch_k(c->pdl, k_u12<32, 2, kSplitBf16>, g, CfgR::THREADS, CfgR::smem(), c->stream, A, lda, K0, knext, n, dinv, bh, nullptr, PW);
             else
-              launch_k(c->pdl, k_u12<32, 2, false>, g, CfgR::THREADS, CfgR::smem(), c->stream, 
-                  A, lda, K0, knext, n, dinv, bh, xsplit ? nullptr : s[3] + (knext - kend) * PW);
+              launch_k(c->pdl, k_u12<32, 2, kSplitTf32>, g, CfgR::THREADS, CfgR::smem(), c->stream, 
+                  A, lda, K0, knext, n, dinv, bh, xsplit ? nullptr : s[3] + (knext - kend) * PW, PW);
             ++c->nlaunch;
             FP_CUDA_TRY(c->err, cudaGetLastError());
           }

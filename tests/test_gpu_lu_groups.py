@@ -1,5 +1,5 @@
 """The static-order factorisation by groups of four panels (lu_static_groups in
-fp_lu_static.cu), from 56 panels on: groups cut short after each panel, ragged last
+fp_lu_static.cu): groups cut short after each panel, ragged last
 panels, against the one by single panels and the residual in FP64."""
 import numpy as np
 import pytest
@@ -7,8 +7,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# 7,192 and 7,200: 24 and 32 columns in a 57th panel; 57 to 60 whole panels
-@pytest.mark.parametrize("nc,ns", [(58, 124), (90, 80), (96, 76), (116, 64), (118, 64), (96, 80)])
+# 7,192 and 7,200: 24 and 32 columns in a 57th panel; 57 to 60 whole panels; then
+# one panel or less, the second begun, one to two groups
+@pytest.mark.parametrize("nc,ns", [(58, 124), (90, 80), (96, 76), (116, 64), (118, 64), (96, 80),
+                                   (10, 10), (16, 8), (12, 12), (16, 16), (20, 14), (32, 16), (34, 16), (40, 24)])
 def test_groups_against_single_panels(fp, nc, ns):
     m = fp.meshes.swept_wing("0012", nc, ns)
     cap = fp._capi
