@@ -544,8 +544,7 @@ def run_ours(args, rank, ws, dist):
     CLm = lift_coefficient(fp, body, x_m, V, U, D, solver)
     CLd = lift_coefficient(fp, body, x_d, V, U, D, solver)
     rel_gamma = float(np.linalg.norm(x_m - x_d) / np.linalg.norm(x_d))
-    # roofline of the dominant kernel of the mixed solve, the tcgen05 3xTF32
-    # trailing update: algorithmic flops (2 m n k per launch) over its summed
+    # roofline of the mixed solve's tcgen05 trailing update from BF16 pairs: algorithmic flops (2 m n k per launch) over its summed
     # per-launch device time in the timed region
     tc_launches, tc_ms, tc_flops, tc_elems = ktime["mixed"]
     tc_tflops = tc_flops / (tc_ms * 1e-3) / 1e12 if tc_ms > 0 else 0.0
@@ -553,10 +552,9 @@ def run_ours(args, rank, ws, dist):
     peak_hbm, hbm_src = measured_peak("hbm_gbs", 6650.0)
     per_elem = profile_traffic("k_tc_gemm_sub")   # DRAM bytes per updated C element, from ncu
     traffic = per_elem * tc_elems / tc_launches if (per_elem and tc_launches) else None
-    # with K = 128 the update does 2 x 128 flops per C element against 8 bytes
-    # of C read-modify-write (32 flop/B), under the ridge point of its BF16
-    # pairs (bf16 peak / 3 MMAs a flop over HBM, ~86 flop/B): HBM is the bound
-    # that applies
+    # the update does 2 x 128 to 2 x 512 flops per C element against 8 bytes of C
+    # read-modify-write (32 to 128 flop/B), about the ridge point of its BF16
+    # pairs (bf16 peak / 3 MMAs a flop over HBM, ~86 flop/B)
     tc_gbs = 8.0 * tc_elems / (tc_ms * 1e-3) / 1e9 if tc_ms > 0 else 0.0
     # the critical path: the panel chain on stream 0, led by the diagonal
     # block (one CTA, dependent elimination steps)
@@ -607,8 +605,8 @@ def run_ours(args, rank, ws, dist):
             "e2e": {"value": e2e_ms, "unit": "ms", "h2d_bytes_per_step": 3 * 8 * N,
                     "d2h_bytes_per_step": 8 * N},
             "gpu_launches": int(launches),
-            "roofline": {"bound": "hbm", "kernel": "k_tc_gemm_sub<2,RED,BF16,X3> (tcgen05 trailing update from BF16 "
-                                                   "hi/lo pairs, three kind::f16 MMAs a 16-deep step, K = 128)",
+            "roofline": {"bound": "hbm", "kernel": "k_tc_x3, k_tc_gemm_sub (tcgen05 trailing update from BF16 hi/lo pairs, "
+                                                   "three kind::f16 MMAs a 16-deep step, K = 128 to 512)",
                          "achieved": tc_gbs, "peak": peak_hbm, "unit": "GB/s", "frac": tc_gbs / peak_hbm,
                          "traffic": traffic, "launches": tc_launches, "ms_total": tc_ms,
                          "algorithmic_bytes": "8 B per updated C element (FP32 read + write; the operand "
@@ -620,7 +618,7 @@ def run_ours(args, rank, ws, dist):
                                          "note": "2 m n k algorithmic flops; the BF16-pair update issues "
                                                  "3 BF16 MMAs per flop"}},
             "critical_path_roofline": None if diag is None else {
-                "bound": "latency", "kernel": "k_pdiag (128 x 128 diagonal block, one CTA)",
+                "bound": "latency", "kernel": "k_pdiag_reg (128 x 128 diagonal block, one CTA)",
                 "avg_us_in_place": diag["avg_us"], "launches": diag["launches"],
                 "achieved_gflops": (2.0 / 3.0) * 128 ** 3 / (diag["avg_us"] * 1e-6) / 1e9,
                 "peak_gflops_one_sm": peak32 * 1e3 / 148.0,
@@ -633,7 +631,7 @@ def run_ours(args, rank, ws, dist):
                                   "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                                   "frac": achieved / peak64,
                                   "peak_source": "measured FP64 FMA throughput (fp_measure_fma_peak)"},
-            "fp64_trailing_update": {"kernel": "k_gemm_sub_dmma<512,4,2,32,2,64,2> (FP64 tensor path, mma.sync .f64, 128 x 64 tiles)",
+            "fp64_trailing_update": {"kernel": "k_i8_gemm_sub (error-free INT8 digits, tcgen05 kind::i8), k_gemm_sub_dmma (narrow updates)",
                                      "launches": d_launches, "ms_total": d_ms,
                                      "tflops": d_flops / (d_ms * 1e-3) / 1e12 if d_ms else 0,
                                      "frac_of_fp64_fma_peak": (d_flops / (d_ms * 1e-3) / 1e12 / peak64) if d_ms else 0,
