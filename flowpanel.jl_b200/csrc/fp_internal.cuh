@@ -112,7 +112,7 @@ struct fp_ctx {
   int panel_gemm = 2;                   // static-order FP32 LU: 1 both panel inverses, GEMM-form L21 / U12; 2: inv(L) only, beside k_l21 (FP_TUNE_PANEL_GEMM)
   bool tc_x3 = true;                    // FP32 form: the update from BF16 pairs, three MMAs (FP_TUNE_TC_BF16X3)
   int tc_prefetch = 1;                  // red.global updates: idle warps prefetch the C tile into L2 (FP_TUNE_TC_PREFETCH)
-  bool lu_split = true;                 // static-order LU: split panel chain (FP_TUNE_LU_SPLIT)
+  bool lu_split = true;                 // static-order LU: split panel chain, groups of panels (FP_TUNE_LU_SPLIT)
   bool l21_async = true;                // static-order LU: k_l21 with asynchronous column-major staging (FP_TUNE_L21_ASYNC)
   bool u12_async = false;               // static-order LU: k_u12g stages A12 column-major by cp.async (FP_TUNE_U12_ASYNC)
   bool u12_wide = false;                // static-order LU: U12 of the columns beyond, 64 columns a CTA (FP_TUNE_U12_WIDE)

@@ -12,12 +12,10 @@
 //
 // Without a pivot search the 128 x 128 diagonal block of a panel is the only
 // sequential work; everything else is tile products:
-//   K1 k_pdiag  one CTA factors the diagonal block in shared memory (32-wide
-//               inner blocks: one warp eliminates a 32 x 32 block in
-//               registers, two warps invert its L and U, all 16 warps form
-//               the inner L / U blocks and the update as register-tiled
-//               products) and keeps the inverses of the four 32 x 32 diagonal
-//               blocks of L and U;
+//   K1 k_pdiag_reg  one CTA factors the diagonal block, 16 warps with 8 columns
+//               each in registers, and forms the inverses of the four 32 x 32
+//               diagonal blocks of L and U (k_pdiag: in shared memory, with
+//               the full inv(L) on request);
 //   K6 k_l21    L21 = A21 U^-1 for the rows below, 64 rows per CTA, by block
 //               substitution with those inverses; writes L21 in place and its
 //               3xTF32 split (hi, lo; K-major) for the tensor-core update;

@@ -475,14 +475,15 @@ int fp_measure_fma_peak(int device, int fp64, double* tflops);
  *                       dependent launch, so that a kernel's launch overlaps
  *                       the end of its stream's previous kernel (12k wing:
  *                       factorisation 11.12 -> 10.79 ms); 0: plain launches
- *   FP_TUNE_LU_SPLIT    1: the panel stream of the static-order LU keeps only
- *                       what the next diagonal block needs (L21 of the next
- *                       panel's rows and the update of its diagonal tile); the
- *                       third stream does L21 of the rows below and the rest of
- *                       the next panel's column beside the next k_pdiag (with
- *                       FP_TUNE_PANEL_GEMM 2; default 1: 12k wing
- *                       factorisation 10.85 -> 10.68 ms); 0: both on the panel
- *                       stream
+ *   FP_TUNE_LU_SPLIT    1 (default; with FP_TUNE_PANEL_GEMM 2): the static-order
+ *                       LU keeps on the panel stream only what the next
+ *                       diagonal block needs and does the rows below on the
+ *                       third stream. The BF16-pair update then goes by groups
+ *                       of four panels, one trailing update a group, unless
+ *                       FP_TUNE_LU_FUSE, REST_SPLIT or PDIAG_LINV is set or
+ *                       FP_TUNE_L21_ASYNC is 0 (12k wing: factorisation 10.5 ->
+ *                       6.7 ms, 36,600 unknowns 219 -> 113); 0: both on the
+ *                       panel stream, an update a panel
  *   FP_TUNE_LU_FUSE     1: with the split chain, U12 of the next panel's
  *                       columns and the update of its diagonal tile (FP32, on
  *                       the FMA pipe) are one kernel; 0 (default): the tile is
