@@ -326,6 +326,7 @@ int gemm_sub_simt_f32(fp_ctx* c, const float* A, const float* B, float* C, int64
                       int kk);
 
 // induced velocity (fp_field.cu)
+int ensure_uind_scratch(fp_ctx* c, size_t n);   // c->d_uscr: n doubles or more
 int launch_uind_ring(fp_ctx* c, const double* d_strength, const double* d_targets, int64_t m,
                      double* d_out, bool fp32);
 int ensure_stage(fp_ctx* c, size_t n);   // the staging buffer holds at least n doubles
