@@ -20,7 +20,9 @@ constexpr int kAsmPanels = 32;     // panels per CTA (smem tile)
 // edges that consecutive panels share are evaluated once (fp_elements.cuh).
 // 12,000 panels with their wake: 2.40 -> 1.89 ms (1.95 with six blocks an SM);
 // with the straight-line reciprocals alone, 2.44: the FP64 pipe is what is busy.
-template <bool W32>
+// Short = false: out of the range of the short forms (fp_elements.cuh), every panel by
+// itself; its own instantiation, since a branch in the kernel costs 3 % there.
+template <bool W32, bool Short>
 __global__ void __launch_bounds__(kAsmThreads, 5)
 k_asm_ring(const PanelRec* __restrict__ panels, int64_t n, const double* __restrict__ tgt,
            int64_t ld, double offset, double cutoff2, double offset2, double* __restrict__ G,
@@ -39,7 +41,8 @@ k_asm_ring(const PanelRec* __restrict__ panels, int64_t n, const double* __restr
   for (int jj = 0; jj < npt; ++jj) {
     const RingPanel<double>& P = sp[jj];
     const int link = jj > 0 ? P.link : 0, next = jj + 1 < npt ? sp[jj + 1].link : 0;
-    const double g = P.nn == 4 ? ring_walk_dot<4>(P, link, next, shared, shared_edge, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2)
+    const double g = !Short    ? ring_dot<double>(P.p, P.nn, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2)
+                     : P.nn == 4 ? ring_walk_dot<4>(P, link, next, shared, shared_edge, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2)
                                : ring_walk_dot<3>(P, link, next, shared, shared_edge, X, Y, Z, n1, n2, n3, offset, cutoff2, offset2);
     const int64_t idx = (j0 + jj) * ld + i;
     G[idx] = g;
@@ -225,10 +228,10 @@ int launch_assemble_ring(fp_ctx* c, double offset, double cutoff, bool write32, 
   cudaStream_t st = s ? s : c->stream;
   dim3 grid((unsigned)((n + kAsmThreads - 1) / kAsmThreads), (unsigned)((n + kAsmPanels - 1) / kAsmPanels));
   const double cut2 = cutoff * cutoff, off2 = offset * offset;
-  if (write32)
-    k_asm_ring<true><<<grid, kAsmThreads, 0, st>>>(c->d_panels, n, c->d_tgt, c->ld, offset, cut2, off2, c->d_G, c->d_G32);
-  else
-    k_asm_ring<false><<<grid, kAsmThreads, 0, st>>>(c->d_panels, n, c->d_tgt, c->ld, offset, cut2, off2, c->d_G, nullptr);
+  const bool fast = c->near_nodes && c->near_tgt && short_forms(offset, cut2);
+  const auto ring = write32 ? (fast ? k_asm_ring<true, true> : k_asm_ring<true, false>)
+                            : (fast ? k_asm_ring<false, true> : k_asm_ring<false, false>);
+  ring<<<grid, kAsmThreads, 0, st>>>(c->d_panels, n, c->d_tgt, c->ld, offset, cut2, off2, c->d_G, write32 ? c->d_G32 : nullptr);
   ++c->nlaunch;
   FP_CUDA_TRY(c->err, cudaGetLastError());
   if (c->nsh > 0) {

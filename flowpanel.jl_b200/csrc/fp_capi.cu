@@ -166,6 +166,7 @@ int fp_ctx_create(int device, fp_ctx** out) {
       cudaMalloc(&c->d_ticket, sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&c->d_p64, 8 * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(c->d_p64, 0, 8 * sizeof(unsigned)) != cudaSuccess ||
+      cudaHostAlloc(&c->h_far, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
       cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->d_ticket, 0, sizeof(unsigned)) != cudaSuccess) {
     delete c;
     return FP_ECUDA;
@@ -187,6 +188,7 @@ int fp_ctx_destroy(fp_ctx* c) {
   dfree(c->d_panels); dfree(c->d_src); dfree(c->d_tgt); dfree(c->d_wake);
   dfree(c->d_geo);
   dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket); dfree(c->d_p64);
+  if (c->h_far) cudaFreeHost(c->h_far);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->ktimer.pool) cudaEventDestroy(e);
@@ -239,8 +241,11 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
         return c->err.set(FP_EINVAL, "fp_set_geometry: node index out of range in panel " + std::to_string(p));
     }
   }
-  for (int64_t i = 0; i < 3 * nnodes; ++i)
+  bool near_nodes = true;
+  for (int64_t i = 0; i < 3 * nnodes; ++i) {
     if (!std::isfinite(nodes[i])) return c->err.set(FP_EINVAL, "fp_set_geometry: non-finite node coordinate");
+    near_nodes = near_nodes && std::fabs(nodes[i]) < kNear;
+  }
   // device buffers only grow: a smaller body reuses them (leading dimension
   // unchanged), so a sequence of bodies allocates for the largest only
   if (npanels > c->capN) {
@@ -249,6 +254,7 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
     c->ld = round_up(npanels, 64);
   }
   c->N = npanels;
+  c->near_nodes = near_nodes;
   c->h_nodes.assign(nodes, nodes + 3 * nnodes);
   c->h_offsets.assign(offsets, offsets + npanels + 1);
   c->h_pnodes.assign(pnodes, pnodes + offsets[npanels]);
@@ -294,7 +300,6 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
   FP_CUDA_TRY(c->err, cudaGetLastError());
   if (int rc = launch_geometry(c, g)) return rc;
   c->h_tgt_valid = false;
-  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));   // the caller may change its arrays (pinned ones too)
   c->has_geometry = true;
   c->nsh = 0;
   c->h_shed.clear();

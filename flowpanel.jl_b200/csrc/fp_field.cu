@@ -45,14 +45,15 @@ k_uind_ring(const PanelRec* __restrict__ panels, const double* __restrict__ stre
   T v = live && !partial ? (T)out[3 * t + 1] : T(0);
   T w = live && !partial ? (T)out[3 * t + 2] : T(0);
   const T off = (T)offset, c2 = (T)cutoff2, o2 = (T)offset2;
-  const bool usual = sizeof(T) == 8 || ordinary_offsets((float)off, (float)c2, (float)o2);
+  const bool usual = sizeof(T) == 8 ? short_forms((double)off, (double)c2) : ordinary_offsets((float)off, (float)c2, (float)o2);
   for (int64_t j0 = jb; j0 < je; j0 += kFieldTile) {
     const int nt = (int)imin64(kFieldTile, je - j0);
     bool near = true;
     __syncthreads();
     for (int q = threadIdx.x; q < nt * 16; q += kFieldThreads)
       near = stage_ring<T>(sp[q / 16], panels[j0 + q / 16], strength[j0 + q / 16], q % 16) && near;
-    const bool ordinary = __syncthreads_and(near) && fabs(X) < T(0x1p20) && fabs(Y) < T(0x1p20) && fabs(Z) < T(0x1p20) && usual;
+    const bool ordinary = __syncthreads_and(near) && fabs(X) < near_limit<T>() && fabs(Y) < near_limit<T>() &&
+                          fabs(Z) < near_limit<T>() && usual;
     if (live) ring_walk(sp, nt, ordinary, X, Y, Z, off, c2, o2, u, v, w);
   }
   if (!live) return;

@@ -30,7 +30,8 @@ __device__ __forceinline__ V3 load3(const double* p) { return {p[0], p[1], p[2]}
 __device__ __forceinline__ void store3(double* p, V3 a) { p[0] = a.x; p[1] = a.y; p[2] = a.z; }
 
 __global__ void __launch_bounds__(128)
-k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* __restrict__ src, double* __restrict__ tgt) {
+k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* __restrict__ src, double* __restrict__ tgt,
+           int* __restrict__ far) {
   const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (p >= n) return;
   const int o0 = a.offsets[p], nn = a.offsets[p + 1] - o0;
@@ -102,6 +103,7 @@ k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* 
     cp = add(add(add(cc, scaled(t, __ddiv_rn(x, (double)nn))), scaled(o, __ddiv_rn(y, (double)nn))),
              scaled(nr, a.cp_offset ? a.cp_offset[p] : 1e-14));
   }
+  if (!near_point(cp.x, cp.y, cp.z)) *far = 1;   // also a NaN: a panel of no extent has no frame
   tgt[p] = cp.x;
   tgt[n + p] = cp.y;
   tgt[2 * n + p] = cp.z;
@@ -113,9 +115,12 @@ k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* 
 }  // namespace
 
 int launch_geometry(fp_ctx* c, const GeometryArgs& g) {
-  k_geometry<<<(unsigned)((c->N + 127) / 128), 128, 0, c->stream>>>(g, c->N, c->d_panels, c->d_src, c->d_tgt);
+  *c->h_far = 0;
+  k_geometry<<<(unsigned)((c->N + 127) / 128), 128, 0, c->stream>>>(g, c->N, c->d_panels, c->d_src, c->d_tgt, c->h_far);
   ++c->nlaunch;
   FP_CUDA_TRY(c->err, cudaGetLastError());
+  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));   // the caller may change its arrays (pinned ones too)
+  c->near_tgt = *c->h_far == 0;
   return FP_OK;
 }
 
