@@ -1305,7 +1305,7 @@ int fp_assembly_vjp(fp_ctx* c, const double* lambda, const double* gamma, const 
   }
   FP_CUDA_TRY(c->err, cudaMemsetAsync(b.gX, 0, b.zero_count * sizeof(double), c->stream));
   if ((rc = launch_vjp_cotangent(c, dl, b.w))) return rc;
-  if ((rc = launch_pair_vjp(c, dg, c->d_tgt, b.w, n, b.gX, b.U, b.gvert, b.gs, b.gwake))) return rc;
+  if ((rc = launch_pair_vjp(c, dg, c->d_tgt, b.w, n, c->near_nodes && c->near_tgt, b.gX, b.U, b.gvert, b.gs, b.gwake))) return rc;
   std::vector<double> hX(3 * n), hU(3 * n), hv(12 * n), hw(kWakeGradHost * c->nsh), hl(n);
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(hX.data(), b.gX, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(hU.data(), b.U, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -1345,8 +1345,10 @@ int fp_uind_vjp(fp_ctx* c, const double* strengths, const double* targets, int64
   if ((rc = vjp_buffers(c, m, b))) return rc;
   // targets and cotangents arrive 3 x m (point-major); the kernels read SoA
   std::vector<double> hx(3 * m), hwv(3 * m);
+  bool near = true;
   for (int64_t i = 0; i < m; ++i)
     for (int d = 0; d < 3; ++d) {
+      near = near && !(std::fabs(targets[3 * i + d]) >= kNear);
       hx[d * m + i] = targets[3 * i + d];
       hwv[d * m + i] = wbar[3 * i + d];
     }
@@ -1355,7 +1357,7 @@ int fp_uind_vjp(fp_ctx* c, const double* strengths, const double* targets, int64
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(b.w, hwv.data(), 3 * m * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(b.gam, strengths, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   FP_CUDA_TRY(c->err, cudaMemsetAsync(b.gX, 0, b.zero_count * sizeof(double), c->stream));
-  if ((rc = launch_pair_vjp(c, b.gam, b.x, b.w, m, b.gX, nullptr, b.gvert, b.gs, b.gwake))) return rc;
+  if ((rc = launch_pair_vjp(c, b.gam, b.x, b.w, m, near, b.gX, nullptr, b.gvert, b.gs, b.gwake))) return rc;
   std::vector<double> hX(3 * m), hv(12 * n), hs(n), hw(kWakeGradHost * c->nsh);
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(hX.data(), b.gX, 3 * m * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   FP_CUDA_TRY(c->err, cudaMemcpyAsync(hv.data(), b.gvert, 12 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

@@ -344,7 +344,7 @@ void post_free(fp_ctx* c);
 
 // reverse mode of the pair kernels (fp_vjp.cu)
 int launch_pair_vjp(fp_ctx* c, const double* d_strength, const double* d_x, const double* d_w,
-                    int64_t m, double* d_gX, double* d_U, double* d_gvert, double* d_gs,
+                    int64_t m, bool near, double* d_gX, double* d_U, double* d_gvert, double* d_gs,
                     double* d_gwake);
 int launch_vjp_cotangent(fp_ctx* c, const double* d_lambda, double* d_w);
 constexpr int kWakeGradHost = 20;   // per shedding edge: pa, pb, qa, qb, da, db, s_pi, s_pj

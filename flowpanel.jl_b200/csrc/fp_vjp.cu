@@ -43,19 +43,28 @@ __device__ __forceinline__ D3 cross3(D3 a, D3 b) {
 __device__ __forceinline__ void acc3(D3& a, D3 b) { a.x += b.x; a.y += b.y; a.z += b.z; }
 
 // Per-node quantities of a target: r = X - p, il = 1/|r| (0 at the node),
-// i = 1/(|r| + offset); roots and reciprocals in straight-line code (near_inv and
-// near_rcp of fp_elements.cuh).
+// i = 1/(|r| + offset). Short: roots and reciprocals in straight-line code (near_inv
+// and near_rcp of fp_elements.cuh, under short_forms() and for coordinates below
+// kNear).
 struct NodeQ { D3 r; double il, i; };
+template <bool Short>
 __device__ __forceinline__ NodeQ nodeq(D3 X, D3 p, double offset) {
   NodeQ q;
   q.r = X - p;
-  q.i = near_inv(dot3(q.r, q.r), offset, q.il);
+  if (Short) {
+    q.i = near_inv(dot3(q.r, q.r), offset, q.il);
+  } else {
+    const double l = sqrt(dot3(q.r, q.r));
+    q.i = 1.0 / (l + offset);
+    q.il = l > 0.0 ? 1.0 / l : 0.0;
+  }
   return q;
 }
 
 // Reverse of one filament edge given its node quantities and r_ab = b - a.
 // Adds df/dr_a to ga, df/dr_b to gb, df/dr_ab to gab, s * U to U and
 // df/ds to gs.
+template <bool Short>
 __device__ __forceinline__ void edge_rev(const NodeQ& A, const NodeQ& B, D3 rab, D3 w, double s,
                                          double cutoff2, double offset2, D3& ga, D3& gb, D3& gab,
                                          D3& U, double& gs) {
@@ -65,14 +74,15 @@ __device__ __forceinline__ void edge_rev(const NodeQ& A, const NodeQ& B, D3 rab,
   const D3 u = A.i * A.r - B.i * B.r;
   const double rd = dot3(rab, u);
   const double den = cc + offset2;
-  const double q = near_rcp(kFourPi * den);
+  const double q = Short ? near_rcp(kFourPi * den) : 1.0 / (kFourPi * den);
   const double g = dot3(c, w);
   const double Arq = rd * q;             // velocity per unit strength is Arq * c
   acc3(U, (s * Arq) * c);
   gs += Arq * g;
   const double Ard = s * g * q;          // df/drd
   const double Ag = s * Arq;             // df/d(c.w)
-  const double Ac = (-2.0 * kFourPi) * q * rd * Ard;   // df/dc via |c|^2, times 1/2 of d|c|^2/dc; 1/den = 4 pi q
+  // df/dc via |c|^2, times 1/2 of d|c|^2/dc; 1/den = 4 pi q
+  const double Ac = Short ? (-2.0 * kFourPi) * q * rd * Ard : -2.0 * s * rd * g * q / den;
   const double ta = A.i * A.i * dot3(rab, A.r) * A.il;
   const double tb = B.i * B.i * dot3(rab, B.r) * B.il;
   acc3(ga, Ard * (A.i * rab - ta * A.r) + Ag * cross3(B.r, w) + Ac * cross3(B.r, c));
@@ -81,18 +91,20 @@ __device__ __forceinline__ void edge_rev(const NodeQ& A, const NodeQ& B, D3 rab,
 }
 
 // Reverse of a free filament pa -> pb of strength s.
+template <bool Short>
 __device__ __forceinline__ void filament_rev(D3 pa, D3 pb, double s, D3 X, D3 w, double offset,
                                              double cutoff2, double offset2, D3& gpa, D3& gpb,
                                              D3& gX, D3& U, double& gs) {
-  const NodeQ A = nodeq(X, pa, offset), B = nodeq(X, pb, offset);
+  const NodeQ A = nodeq<Short>(X, pa, offset), B = nodeq<Short>(X, pb, offset);
   D3 ga = d3(0, 0, 0), gb = d3(0, 0, 0), gab = d3(0, 0, 0);
-  edge_rev(A, B, pb - pa, w, s, cutoff2, offset2, ga, gb, gab, U, gs);
+  edge_rev<Short>(A, B, pb - pa, w, s, cutoff2, offset2, ga, gb, gab, U, gs);
   acc3(gX, ga + gb);
   gpa = gpa - ga - gab;
   gpb = gpb - gb + gab;
 }
 
 // Reverse of the semi-infinite vortex from p along d (strength s).
+template <bool Short>
 __device__ __forceinline__ void semiinf_rev(D3 p, D3 d, double s, D3 X, D3 w, double offset,
                                             double cutoff2, double offset2, D3& gp, D3& gd, D3& gX,
                                             D3& U, double& gs) {
@@ -101,7 +113,7 @@ __device__ __forceinline__ void semiinf_rev(D3 p, D3 d, double s, D3 X, D3 w, do
   const D3 p0 = p + t * d;
   const D3 e = p0 - p;
   D3 gp0 = d3(0, 0, 0);
-  if (dot3(e, e) > offset2) filament_rev(p, p0, s, X, w, offset, cutoff2, offset2, gp, gp0, gX, U, gs);
+  if (dot3(e, e) > offset2) filament_rev<Short>(p, p0, s, X, w, offset, cutoff2, offset2, gp, gp0, gX, U, gs);
   const D3 h = X - p0;
   const double hsqr = dot3(h, h);
   if (hsqr > cutoff2) {
@@ -124,13 +136,13 @@ __device__ __forceinline__ void semiinf_rev(D3 p, D3 d, double s, D3 X, D3 w, do
 
 // Reverse of a ring of NN nodes (one pair): vertex gradients into gv, the
 // target gradient and velocity into gX, U, df/ds into gs.
-template <int NN>
+template <int NN, bool Short>
 __device__ __forceinline__ void ring_rev(const double* __restrict__ p, double s, D3 X, D3 w,
                                          double offset, double cutoff2, double offset2, D3* gv,
                                          D3& gX, D3& U, double& gs) {
   NodeQ q[NN];
 #pragma unroll
-  for (int k = 0; k < NN; ++k) q[k] = nodeq(X, d3(p[3 * k], p[3 * k + 1], p[3 * k + 2]), offset);
+  for (int k = 0; k < NN; ++k) q[k] = nodeq<Short>(X, d3(p[3 * k], p[3 * k + 1], p[3 * k + 2]), offset);
   D3 gr[NN];
 #pragma unroll
   for (int k = 0; k < NN; ++k) gr[k] = d3(0, 0, 0);
@@ -139,7 +151,7 @@ __device__ __forceinline__ void ring_rev(const double* __restrict__ p, double s,
     const int b = (a + 1) % NN;
     const D3 rab = d3(p[3 * b] - p[3 * a], p[3 * b + 1] - p[3 * a + 1], p[3 * b + 2] - p[3 * a + 2]);
     D3 gab = d3(0, 0, 0);
-    edge_rev(q[a], q[b], rab, w, s, cutoff2, offset2, gr[a], gr[b], gab, U, gs);
+    edge_rev<Short>(q[a], q[b], rab, w, s, cutoff2, offset2, gr[a], gr[b], gab, U, gs);
     acc3(gv[b], gab);
     gv[a] = gv[a] - gab;
   }
@@ -190,6 +202,7 @@ constexpr int kVjpChunk = 512;     // targets per CTA
 // FP64 pipe: 6,300 x 6,300 pairs 3.23 -> 2.19 ms with one reciprocal an edge instead
 // of four divisions and one root a node (2.35 with 128 registers and four CTAs an SM
 // instead of three).
+template <bool Short>
 __global__ void __launch_bounds__(kVjpThreads)
 k_vjp_ring(const PanelRec* __restrict__ panels, const double* __restrict__ strength, int64_t n,
            const double* __restrict__ tx, const double* __restrict__ tw, int64_t m, double offset,
@@ -234,8 +247,8 @@ k_vjp_ring(const PanelRec* __restrict__ panels, const double* __restrict__ stren
       const D3 w = d3(st[t][3], st[t][4], st[t][5]);
       D3 gx = d3(0, 0, 0), U = d3(0, 0, 0);
       if (valid) {
-        if (nn == 4) ring_rev<4>(p, s, X, w, offset, cutoff2, offset2, gv, gx, U, gs);
-        else ring_rev<3>(p, s, X, w, offset, cutoff2, offset2, gv, gx, U, gs);
+        if (nn == 4) ring_rev<4, Short>(p, s, X, w, offset, cutoff2, offset2, gv, gx, U, gs);
+        else ring_rev<3, Short>(p, s, X, w, offset, cutoff2, offset2, gv, gx, U, gs);
       }
       const double v[8] = {gx.x, gx.y, gx.z, U.x, U.y, U.z, 0.0, 0.0};
       const double r = warp_reduce_scatter8(v, lane);
@@ -272,6 +285,7 @@ constexpr int kVjpWakeThreads = 128;
 constexpr int kWakeEdges = 8;
 constexpr int kWakeGrad = 20;   // pa, pb, qa, qb, da, db (3 each), s_pi, s_pj
 
+template <bool Short>
 __global__ void __launch_bounds__(kVjpWakeThreads)
 k_vjp_wake(const WakeRec* __restrict__ wake, int64_t nsh, const double* __restrict__ strength,
            const double* __restrict__ tx, const double* __restrict__ tw, int64_t m, double offset,
@@ -299,9 +313,9 @@ k_vjp_wake(const WakeRec* __restrict__ wake, int64_t nsh, const double* __restri
       // (U_semiinfinite_horseshoe, src/FLOWPanel_elements.jl:692-730)
       const double si = strength[R.pi];
       double g1 = 0.0, g2 = 0.0, g3 = 0.0;
-      semiinf_rev(pa, da, -si, X, w, offset, cutoff2, offset2, gpa, gda, gx, U, g1);
-      filament_rev(pa, pb, si, X, w, offset, cutoff2, offset2, gpa, gpb, gx, U, g2);
-      semiinf_rev(pb, db, si, X, w, offset, cutoff2, offset2, gpb, gdb, gx, U, g3);
+      semiinf_rev<Short>(pa, da, -si, X, w, offset, cutoff2, offset2, gpa, gda, gx, U, g1);
+      filament_rev<Short>(pa, pb, si, X, w, offset, cutoff2, offset2, gpa, gpb, gx, U, g2);
+      semiinf_rev<Short>(pb, db, si, X, w, offset, cutoff2, offset2, gpb, gdb, gx, U, g3);
       gsi = -g1 + g2 + g3;
       if (R.pj >= 0) {
         // lower side: its own TE nodes with the directions swapped (db, da)
@@ -309,9 +323,9 @@ k_vjp_wake(const WakeRec* __restrict__ wake, int64_t nsh, const double* __restri
         const D3 qa = d3(R.qa[0], R.qa[1], R.qa[2]), qb = d3(R.qb[0], R.qb[1], R.qb[2]);
         const double sj = strength[R.pj];
         double h1 = 0.0, h2 = 0.0, h3 = 0.0;
-        semiinf_rev(qa, db, -sj, X, w, offset, cutoff2, offset2, gqa, gdb, gx, U, h1);
-        filament_rev(qa, qb, sj, X, w, offset, cutoff2, offset2, gqa, gqb, gx, U, h2);
-        semiinf_rev(qb, da, sj, X, w, offset, cutoff2, offset2, gqb, gda, gx, U, h3);
+        semiinf_rev<Short>(qa, db, -sj, X, w, offset, cutoff2, offset2, gqa, gdb, gx, U, h1);
+        filament_rev<Short>(qa, qb, sj, X, w, offset, cutoff2, offset2, gqa, gqb, gx, U, h2);
+        semiinf_rev<Short>(qb, da, sj, X, w, offset, cutoff2, offset2, gqb, gda, gx, U, h3);
         gsj = -h1 + h2 + h3;
       }
     }
@@ -354,22 +368,25 @@ __global__ void k_vjp_cotangent(const double* __restrict__ lambda, const double*
 // Gradient of F = sum_i w_i . sum_j s_j U_j(X_i) over the body's rings and
 // wake horseshoes. All outputs are accumulated (the caller zeroes them):
 // gX, U 3 x m (SoA), gvert N x 12 (per panel, node k at 3k..3k+2), gs N,
-// gwake nsh x 20.
+// gwake nsh x 20. near: every target is below kNear in size (or NaN, which no edge counts).
 int launch_pair_vjp(fp_ctx* c, const double* d_strength, const double* d_x, const double* d_w,
-                    int64_t m, double* d_gX, double* d_U, double* d_gvert, double* d_gs,
+                    int64_t m, bool near, double* d_gX, double* d_U, double* d_gvert, double* d_gs,
                     double* d_gwake) {
   const int64_t n = c->N;
   const double offset = c->kern_offset, cut2 = c->kern_cutoff * c->kern_cutoff, off2 = offset * offset;
   dim3 g((unsigned)((n + kVjpThreads - 1) / kVjpThreads), (unsigned)((m + kVjpChunk - 1) / kVjpChunk));
-  k_vjp_ring<<<g, kVjpThreads, 0, c->stream>>>(c->d_panels, d_strength, n, d_x, d_w, m, offset, cut2, off2,
-                                               d_gX, d_U, d_gvert, d_gs);
+  const bool fast = near && c->near_nodes && short_forms(offset, cut2);
+  const auto ring = fast ? k_vjp_ring<true> : k_vjp_ring<false>;
+  const auto wake = fast ? k_vjp_wake<true> : k_vjp_wake<false>;
+  ring<<<g, kVjpThreads, 0, c->stream>>>(c->d_panels, d_strength, n, d_x, d_w, m, offset, cut2, off2, d_gX, d_U, d_gvert,
+                                         d_gs);
   ++c->nlaunch;
   FP_CUDA_TRY(c->err, cudaGetLastError());
   if (c->nsh > 0) {
     dim3 g2((unsigned)((m + kVjpWakeThreads - 1) / kVjpWakeThreads),
             (unsigned)((c->nsh + kWakeEdges - 1) / kWakeEdges));
-    k_vjp_wake<<<g2, kVjpWakeThreads, 0, c->stream>>>(c->d_wake, c->nsh, d_strength, d_x, d_w, m, offset, cut2,
-                                                      off2, d_gX, d_U, d_gwake);
+    wake<<<g2, kVjpWakeThreads, 0, c->stream>>>(c->d_wake, c->nsh, d_strength, d_x, d_w, m, offset, cut2, off2, d_gX, d_U,
+                                                d_gwake);
     ++c->nlaunch;
     FP_CUDA_TRY(c->err, cudaGetLastError());
   }

@@ -74,3 +74,38 @@ def test_degenerate_panel_is_refused(fp, kind, precision):
     with pytest.raises(fp._capi.FlowPanelError, match="zero pivot"):
         fp.solve(body, np.tile(V, (m.npanels, 1)), D, D, solver=solver)
     solver.close()
+
+
+def _vjp(ctx, m, g, X, W, offset=1e-8):
+    ctx.set_geometry(m.nodes, m.panel_offsets, m.panel_nodes)
+    ctx.assemble(1, offset)
+    return ctx.uind_vjp(g, X, W, m.nnodes)
+
+
+def test_reverse_mode_of_far_targets(fp, ctx):
+    """Targets whose cross products overflow or are not numbers add nothing to
+    the gradient of an ordinary one."""
+    m = _sphere(fp)
+    rng = np.random.default_rng(8)
+    g, W = rng.standard_normal(m.npanels), rng.standard_normal((4, 3))
+    X = np.array([[1.7, 0.4, -0.3], [1e90, 1e90, 1e90], [np.nan, 0, 0], [-1e95, 2e95, 1e94]])
+    one, all_ = _vjp(ctx, m, g, X[:1], W[:1]), _vjp(ctx, m, g, X, W)
+    assert (all_["dtargets"][1:] == 0.0).all()
+    for k in ("dnodes", "dstrengths"):   # the same terms, added in another order
+        assert np.abs(all_[k] - one[k]).max() < 1e-14 * np.abs(one[k]).max()
+    assert np.abs(all_["dtargets"][0] - one["dtargets"][0]).max() < 1e-14 * np.abs(one["dtargets"]).max()
+
+
+@pytest.mark.parametrize("offset,scale", [(-1e-8, 1.0), (0.0, 1.0), (1e-8, 2.0 ** 61), (1e-8, 2.0 ** 59)])
+def test_reverse_mode_out_of_range(fp, O, ctx, offset, scale):
+    """Against the oracle's Dual numbers, to the bound of test_gpu_adjoint.py."""
+    m = _sphere(fp, scale)
+    rng = np.random.default_rng(9)
+    g = rng.standard_normal(m.npanels)
+    X = scale * np.concatenate([1.1 * rng.standard_normal((40, 3)), m.nodes[:4] / scale + 1e-3 * rng.standard_normal((4, 3))])
+    W = rng.standard_normal(X.shape)
+    got = _vjp(ctx, m, g, X, W, offset)
+    for key in ("dnodes", "dtargets", "dstrengths"):
+        v = rng.standard_normal(got[key].shape)
+        _, dF = O.uind_jvp(m, g, NONE, NONE, X, W, offset=offset, **{key: v})
+        assert abs(np.sum(got[key] * v) - dF) <= 1e-9 * np.sum(np.abs(got[key] * v))
