@@ -111,9 +111,7 @@ void free_matrices(fp_ctx* c) {
   for (int s = 0; s < 2; ++s) {
     for (int i = 0; i < 4; ++i) dfree(c->d_tc[s][i]);
     c->tc_cap[s] = 0;
-    dfree(c->d_i8[s]);
   }
-  c->i8_cap = 0;
   c->cap_rhs = 0; c->cap_gmres_m = 0;
   c->assembled = -1; c->factored = -1; c->nrhs = 0;
   if (c->lu_graph) cudaGraphExecDestroy(c->lu_graph);

@@ -186,8 +186,6 @@ struct fp_ctx {
   float* d_tc[2][4] = {{nullptr, nullptr, nullptr, nullptr}, {nullptr, nullptr, nullptr, nullptr}};
   size_t tc_cap[2] = {0, 0};
   int tc_slot = 0;                      // scratch set of the current launches
-  uint8_t* d_i8[2] = {nullptr, nullptr};   // FP64 LU: 8-bit digits and scales of a panel's operands, by panel parity
-  int64_t i8_cap = 0;                      // rows (and columns) they hold
   cudaStream_t stream2 = nullptr;       // second stream of the look-ahead factorisation
   cudaStream_t stream3 = nullptr;       // third stream (high priority): the static-order LU's inv(L) beside k_l21
   cudaStream_t stream4 = nullptr;       // fourth stream (high priority): U12 of the columns beyond, beside the trailing update
@@ -302,13 +300,6 @@ bool tc_gemm_sub_bf16(fp_ctx* c, const void* Ah, const void* Bh, int ldk, float*
                       int64_t nn, int kk);
 bool tc_gemm_sub_bf16x3(fp_ctx* c, const void* Ah, const void* Al, const void* Bh, const void* Bl, int ldk, float* C,
                         int64_t ldc, int64_t m, int64_t nn, int kk);
-// FP64 trailing update on the INT8 tensor cores (fp_i8.cu): scratch for n
-// rows, the digits of a panel's m rows of L (set: panel parity), and the
-// update of n columns, col0 columns right of the panel (the digits of their
-// U rows B are formed first); K = kOuterPanel
-int i8_scratch(fp_ctx* c, int64_t n);
-int i8_slice_rows(fp_ctx* c, int set, const double* A, int64_t lda, int64_t m);
-int i8_gemm_sub(fp_ctx* c, int set, const double* B, double* C, int64_t ld, int64_t m, int64_t col0, int64_t n);
 // b = FP32 copy of the FP64 a rounded to BF16 values
 int convert_f64_bf16(fp_ctx* c, const double* a, float* b, int64_t n, int64_t k, int64_t lda, int64_t ldb);
 // FP32 trailing update on tensor cores (fp_tc.cu); returns false if the

@@ -4,8 +4,7 @@
 //
 // Per panel: k_panel64 factors its columns in one launch; k_strip64 swaps the
 // panel's rows and forms U12 in the columns beside it; the trailing update
-// follows on the INT8 tensor cores (fp_i8.cu) or the FP64 tensor path
-// (fp_lu.cu), the next panel's columns first.
+// follows on the FP64 tensor path (fp_lu.cu), the next panel's columns first.
 //
 // The panel is a chain of 256 dependent pivot steps, so its kernels are built
 // for latency: one CTA of 16 warps holds 64 rows of the panel in shared memory
@@ -623,14 +622,11 @@ k_strip64(double* __restrict__ A, int64_t lda, int64_t K0, int w, const double* 
 // Row swaps stay inside 64-row blocks, so the swaps of different blocks
 // commute, and a row update commutes with a swap of the rows of both C and L.
 //
-// Panels with kI8Rows rows below them update on the INT8 tensor cores
-// (fp_i8.cu) unless a variant of FP_TUNE_FP64_DMMA is asked for. Below that
-// the digits' two launches and a tile's latency (35 us) cost what the INT8
-// update saves. Factorisation with the digits from 512 rows on, from 2,048 on
-// and never: 1,840 unknowns 1.56, 1.52, 1.55 ms; 3,000 2.59, 2.57, 2.58; 4,200
-// 3.78, 3.78, 4.16; 6,300 7.35, 7.34, 9.23; 12,000 31.1, 31.2, 47.4.
-constexpr int64_t kI8Rows = 2048;
-
+// The update's products stay in FP64: as seven INT8 digits under a scale a row and
+// column (exact sums on the INT8 tensor cores) it took 31 ms of a factorisation of
+// 12,000 where this takes 47, but an entry loses the bits by which it lies below its
+// row's largest. The factors' error was 1e-9 of |L||U| in places (here 4e-15), and
+// the response of one of two bodies to the other held 9 digits instead of 15.
 template <>
 int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipiv, float* cert) {
   constexpr int W = p64::W, R = p64::R;
@@ -641,9 +637,6 @@ int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipi
   FP_CUDA_TRY(c->err, attr_panel.ensure(p64::k_panel64, (int)p64::kSmem));
   FP_CUDA_TRY(c->err, attr_strip.ensure(p64::k_strip64, (int)p64::strip::kSmem));
   static_assert(W / R <= kPanelSlots && 8 * p64::SUB * p64::SUB <= p64::SLOT, "one scratch slot per block of a panel");
-  const bool i8 = c->fp64_dmma == 6 && n >= W + kI8Rows;
-  if (i8)
-    if (int rc = i8_scratch(c, n)) return rc;
   // the blocks' inverses and row orders, two sets (panel parity): stream2's
   // strip of panel P reads its set while panel P + 1 fills the other
   double* const slots0 = reinterpret_cast<double*>(c->d_minv);
@@ -659,7 +652,6 @@ int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipi
     const int set = (int)((K0 / W) & 1), w = (int)(kend - K0);
     double* const slots = slots0 + (size_t)set * kPanelSlots * p64::SLOT;
     int* const rowat = rowat0 + (size_t)set * kPanelSlots * R;
-    const bool digits = i8 && n - kend >= kI8Rows;
     {
       const unsigned ctas = (unsigned)((n - K0 + R - 1) / R);
       TraceScope tr(c, TR_L21);
@@ -670,8 +662,6 @@ int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipi
       c->p64_ticket += ctas;
       c->p64_flag += 8;   // more than the levels a block publishes
     }
-    if (digits)
-      if (int rc = i8_slice_rows(c, set, at(kend, K0), lda, n - kend)) return rc;
     FP_CUDA_TRY(c->err, cudaEventRecord(c->ev_panel, c->stream));
     auto strip = [&](int64_t cl0, int64_t cl1, int64_t cr0, int64_t cr1) -> int {
       const int64_t g = (cl1 - cl0 + p64::strip::COLS - 1) / p64::strip::COLS +
@@ -686,7 +676,6 @@ int lu_factor<double>(fp_ctx* c, double* A, int64_t n, int64_t lda, int32_t* ipi
     };
     // columns [c0, c1) right of the panel -= L21 U12
     auto update = [&](int64_t c0, int64_t c1) -> int {
-      if (digits) return i8_gemm_sub(c, set, at(K0, c0), at(kend, c0), lda, n - kend, c0 - kend, c1 - c0);
       return gemm_sub_f64(c, at(kend, K0), at(K0, c0), at(kend, c0), lda, n - kend, c1 - c0, w);
     };
     if (knext > kend) {

@@ -412,10 +412,7 @@ int fp_measure_fma_peak(int device, int fp64, double* tflops);
  *                       slices (20.8); on 128 x 64 tiles, two CTAs of 16 warps
  *                       an SM: 5 with 16-deep slices in 3 stages (22.4), 6
  *                       (default) with 32-deep slices in 2 stages (23.1);
- *                       all give the same results. With the default, panels
- *                       of at least 2,048 rows below update on the INT8
- *                       tensor cores instead, from an error-free split into
- *                       8-bit digits, as accurate as the FP64 products
+ *                       all give the same results
  *   FP_TUNE_TC_SPLIT    the static-order LU's tensor-core update: 0 reads
  *                       operands split into TF32 hi / lo by the panel kernels
  *                       (32 KB a K block); 1, 2, 3: reads the unsplit FP32
