@@ -43,10 +43,13 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, int bytes) {
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// waits (bounded) for a pivot step's barrier
-__device__ __forceinline__ void wait_step(uint64_t* bar) {
+// waits for a pivot step's barrier, kStepTries at most, and adds the tries' bits to
+// `late` (the caller goes on, with the identity as the row order; see step_status)
+constexpr int kStepTries = 1 << 16;
+__device__ __forceinline__ void wait_step(uint64_t* bar, int& late) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);
-  for (int i = 0; i < (1 << 16); ++i) {
+  int i = 0;
+  for (; i < kStepTries; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -57,7 +60,11 @@ __device__ __forceinline__ void wait_step(uint64_t* bar) {
         : "memory");
     if (ok) break;
   }
+  late |= i;
   __syncwarp();
+}
+__device__ __forceinline__ void step_status(int late, int* status) {   // after a warp's last wait
+  if (late & kStepTries) atomicOr(status, (int)DEV_TIMEOUT);
 }
 
 struct Smem {
@@ -65,8 +72,8 @@ struct Smem {
   double (*Q)[R][PP];   // two 64 x 64 operands, [column][row]
   double* VU;           // inverses of the block's 16 x 16 U sub-blocks, [q][column][k]
   double* VL;           // of its L sub-blocks, [q][k][row]
-  int* pr;              // physical row of each logical row
-  int* lp;              // logical position of each step's pivot
+  int* pr;              // physical row of each logical row (until the block is factored: the identity)
+  int* lp;              // logical position of each step's pivot (the same)
   uint64_t* step;       // one barrier a pivot step: its column and pivot row are written
   int* stop;
 };
@@ -153,6 +160,7 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
     a1[c] = D[own + c][lane + 32];
   }
   bool used0 = false, used1 = false, zero = false;
+  int late = 0;
   int pos0 = lane, pos1 = lane + 32;
   // the pivot row of step J takes logical place J, the row that had it the pivot's
   auto take = [&](int J, int pr, int lpos) {
@@ -161,7 +169,7 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
   };
 #pragma unroll 1
   for (int J = 0; J < own; ++J) {
-    wait_step(s.step + J);
+    wait_step(s.step + J, late);
     const int pr = s.pr[J], src = pr & 31;
     const double l0 = D[J][lane], l1 = D[J][lane + 32];
     take(J, pr, s.lp[J]);
@@ -239,11 +247,12 @@ __device__ __forceinline__ void factor_diag(Smem& s, double (*D)[PP], int nb, do
   // the inverses of the sub-blocks, as each is done
   if (warp < 8) {
     const int J0 = (warp >> 1) * SUB;
-    wait_step(s.step + J0 + SUB - 1);
+    wait_step(s.step + J0 + SUB - 1, late);
     auto rowof = [&](int r) { return s.pr[r]; };
     if (warp & 1) inv_upper(s, D, J0, lane, rowof);
     else inv_lower(s, D, J0, lane, rowof);
   }
+  step_status(late, status);
   __syncthreads();
   double (*L)[PP] = s.Q[0];
   for (int e = tid; e < R * R; e += NT) {
@@ -399,6 +408,7 @@ k_panel64(double* __restrict__ A, int64_t lda, int64_t n, int64_t K0, int w, int
   __syncthreads();
   const int c = s.lp[0];
   __syncthreads();
+  if (tid < R) s.pr[tid] = s.lp[tid] = tid;   // what a CTA that gives up leaves as its row order and pivots
   const int64_t r0 = K0 + (int64_t)c * R;
   const int rows = (int)imin64(R, n - r0);
   const int nblk = (w + R - 1) / R;
