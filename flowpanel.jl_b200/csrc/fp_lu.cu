@@ -1958,14 +1958,14 @@ static int run_trs(fp_ctx* c, const T* A, int64_t n, int64_t lda, const T* Dinv,
   return FP_OK;
 }
 
-template <class T>
+template <class T, bool TRANS>
 static int solve_group(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const T* Dinv, T* B,
                        int64_t ldb, int kr) {
   int rc;
 #define FP_TRS_CASE(KR)                                                               \
   case KR:                                                                            \
-    if ((rc = run_trs<T, true, KR, true>(c, LU, n, lda, Dinv, B, ldb))) return rc;    \
-    return run_trs<T, false, KR, true>(c, LU, n, lda, Dinv, B, ldb);
+    if ((rc = run_trs<T, true, KR, TRANS>(c, LU, n, lda, Dinv, B, ldb))) return rc;   \
+    return run_trs<T, false, KR, TRANS>(c, LU, n, lda, Dinv, B, ldb);
   switch (kr) {
     FP_TRS_CASE(1)
     FP_TRS_CASE(2)
@@ -1990,7 +1990,7 @@ int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv
     for (int64_t q0 = 0; q0 < k;) {
       const int64_t left = k - q0;
       const int kr = left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
-      int rc = solve_group<T>(c, LU, n, lda, Dinv, B + q0 * ldb, ldb, kr);
+      int rc = solve_group<T, true>(c, LU, n, lda, Dinv, B + q0 * ldb, ldb, kr);
       if (rc) return rc;
       q0 += kr;
     }
@@ -2007,10 +2007,18 @@ int lu_solve(fp_ctx* c, const T* LU, int64_t n, int64_t lda, const int32_t* ipiv
     ++c->nlaunch;
     FP_CUDA_TRY(c->err, cudaGetLastError());
   }
+  // two right-hand sides of a small system, and four in FP64: one sweep over 64-row
+  // blocks (k_trs). FP64, two: 480 unknowns 61 us against 82 for two sweeps by k_trs1,
+  // 1,020 465 against 495, 2,000 203 against 196; FP32 refinement 288 against 322, 406
+  // against 402, 675 against 577. Four in FP64: 2,000 272 us against 288 for k_trsm, 8,000
+  // 1,067 against 1,083, 12,000 1,632 against 1,607; in FP32 k_trsm wins from 480 on.
+  if ((k == 2 && n <= 1024) || (k == 4 && sizeof(T) == 8 && n <= 8192))
+    return solve_group<T, false>(c, LU, n, lda, Dinv, B, ldb, (int)k);
   const T* D128 = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_dinv128_64 : (void*)c->d_dinv128_32);
   const T* Mp = reinterpret_cast<const T*>(sizeof(T) == 8 ? (void*)c->d_mprev64 : (void*)c->d_mprev32);
   // one right-hand side, or two in turn: the 128-row streaming sweeps (FP64, n =
-  // 12,000: 0.53 ms each against 1.58 ms for k_trsm's least group)
+  // 12,000: 0.53 ms each against 1.58 ms for k_trsm's least group; FP32 refinement of two
+  // 4.1 ms against 5.3 for three by k_trsm)
   if (k <= 2) {
     static SmemAttr attr_lo, attr_up;
     FP_CUDA_TRY(c->err, attr_lo.ensure(k_trs1<T, true>, (int)trs1_smem<T>()));
