@@ -17,6 +17,7 @@
 // host synchronisation and plain loads a step took 236 us.
 #include <cmath>
 #include <cstring>
+#include <string>
 #include <vector>
 
 #include "fp_internal.cuh"
@@ -269,18 +270,25 @@ constexpr int kAhead = 2, kRing = kAhead + 1;
 int ensure_basis(fp_ctx* c, int cap, int keep) {
   if (c->cap_gmres_m >= cap) return FP_OK;
   const int64_t ld = c->ld;
+  for (cudaEvent_t& ev : c->ev_gm)
+    if (!ev) FP_CUDA_TRY(c->err, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   double* V = nullptr;
   double* h = nullptr;
   double* ring = nullptr;
-  FP_CUDA_TRY(c->err, cudaHostAlloc(&ring, (size_t)kRing * (cap + 2) * sizeof(double), cudaHostAllocMapped));
-  for (cudaEvent_t& e : c->ev_gm)
-    if (!e) FP_CUDA_TRY(c->err, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  FP_CUDA_TRY(c->err, cudaMalloc(&V, (size_t)(cap + 3) * ld * sizeof(double)));
-  FP_CUDA_TRY(c->err, cudaMalloc(&h, (size_t)(3 * (cap + 1) + 16) * sizeof(double)));
-  if (c->d_V && keep > 0)
-    FP_CUDA_TRY(c->err, cudaMemcpyAsync(V, c->d_V, (size_t)keep * ld * sizeof(double), cudaMemcpyDeviceToDevice,
-                                        c->stream));
-  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));
+  // the basis first: if there is no room for it, no host memory is pinned
+  cudaError_t e = cudaMalloc(&V, (size_t)(cap + 3) * ld * sizeof(double));
+  if (!e) e = cudaMalloc(&h, (size_t)(3 * ((size_t)cap + 1) + 16) * sizeof(double));
+  if (!e) e = cudaHostAlloc(&ring, (size_t)kRing * ((size_t)cap + 2) * sizeof(double), cudaHostAllocMapped);
+  if (!e && c->d_V && keep > 0)
+    e = cudaMemcpyAsync(V, c->d_V, (size_t)keep * ld * sizeof(double), cudaMemcpyDeviceToDevice, c->stream);
+  if (!e) e = cudaStreamSynchronize(c->stream);
+  if (e) {
+    cudaFree(V);
+    cudaFree(h);
+    if (ring) cudaFreeHost(ring);
+    cudaGetLastError();
+    return c->err.set(FP_ECUDA, std::string("GMRES basis: ") + cudaGetErrorString(e));
+  }
   if (c->d_V) cudaFree(c->d_V);
   if (c->d_h) cudaFree(c->d_h);
   if (c->h_gm) {
