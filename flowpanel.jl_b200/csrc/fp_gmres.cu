@@ -405,7 +405,8 @@ int gmres_solve(fp_ctx* c, const double* b, double* x, int64_t k, const fp_solve
       const int64_t steps = std::min<int64_t>(restart ? mem : itmax, itmax - it);
       int queued = 0;
       for (int j = 0; j < steps; ++j) {
-        for (; queued <= j + ahead && queued < steps; ++queued)
+        // ahead only in the basis there is: it grows for a step that is taken
+        for (; queued < steps && (queued == j || (queued <= j + ahead && queued + 1 <= c->cap_gmres_m)); ++queued)
           if (int rc = launch(queued)) return rc;
         FP_CUDA_TRY(c->err, cudaEventSynchronize(c->ev_gm[j % kRing]));
         const double* hj = c->h_gm + (size_t)(j % kRing) * (c->cap_gmres_m + 2);

@@ -1,4 +1,5 @@
-"""The Krylov basis of GMRES (fp_gmres.cu): one there is no room for is refused."""
+"""The Krylov basis of GMRES (fp_gmres.cu): it grows for a step that is taken, not for
+one launched ahead, and a basis there is no room for is refused."""
 import numpy as np
 import pytest
 
@@ -20,6 +21,26 @@ def _setup(fp, nc, ns):
 def _solve(fp, c, U, memory, itmax=0):
     opts = fp._capi.make_opts("gmres", "fp64", gmres_memory=memory, gmres_atol=1e-10, gmres_rtol=1e-10, gmres_itmax=itmax)
     return c.solve_body(fp._capi.FP_ELEMENT_VORTEXRING, U, opts=opts)
+
+
+def test_basis_does_not_grow_for_steps_ahead(fp):
+    """Device memory of a solve of `steps` steps with room for exactly those and with
+    room for the two launched ahead: a basis that doubled would hold 5 MB or more on top."""
+    torch = pytest.importorskip("torch")
+    used, xs = [], []
+    c, U = _setup(fp, 46, 90)
+    x, st = _solve(fp, c, U, 1000)
+    c.close()
+    steps = st.gmres_iters
+    assert 150 < steps < 998   # doubling the basis: steps x 33 KB, 5 MB or more
+    for memory in (steps + 2, steps):
+        free0 = torch.cuda.mem_get_info()[0]
+        c, U = _setup(fp, 46, 90)
+        y, st = _solve(fp, c, U, memory)
+        used.append(free0 - torch.cuda.mem_get_info()[0])
+        c.close()
+        assert st.gmres_iters == steps and (y == x).all()
+    assert abs(used[1] - used[0]) <= 4 << 20   # the allocator's granularity, 2 MB a buffer
 
 
 def test_basis_without_room(fp):
