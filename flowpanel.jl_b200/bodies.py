@@ -161,7 +161,7 @@ def _panel_arrays(mesh: Mesh):
     offs = mesh.panel_offsets
     nn = np.diff(offs)
     idx = np.zeros((mesh.npanels, 4), np.int64)
-    if nn.size and (nn == nn[0]).all():
+    if nn.size and nn[0] in (3, 4) and (nn == nn[0]).all():
         idx[:, :nn[0]] = np.reshape(mesh.panel_nodes[offs[0]:offs[-1]], (-1, nn[0]))
         return idx, nn
     for k in range(4):
