@@ -52,3 +52,19 @@ def test_basis_without_room(fp):
     x, st = _solve(fp, c, U, 50)
     assert st.gmres_iters > 0 and np.isfinite(x).all()
     c.close()
+
+
+def test_breakdown_with_steps_ahead(fp):
+    """A tolerance of zero on 16 unknowns: the Krylov space is exhausted while later
+    steps are under way. The process ends unconverged, and the context's next solve
+    is that of a new one."""
+    c, U = _setup(fp, 4, 4)
+    with pytest.raises(fp._capi.FlowPanelError, match="did not reach its tolerance"):
+        c.solve_body(fp._capi.FP_ELEMENT_VORTEXRING, U,
+                     opts=fp._capi.make_opts("gmres", "fp64", gmres_memory=3, gmres_atol=0.0, gmres_rtol=0.0))
+    x, st = _solve(fp, c, U, 50)
+    c.close()
+    c, U = _setup(fp, 4, 4)
+    y, sy = _solve(fp, c, U, 50)
+    c.close()
+    assert (x == y).all() and st.gmres_iters == sy.gmres_iters
