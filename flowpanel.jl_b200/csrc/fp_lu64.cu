@@ -89,18 +89,6 @@ __device__ __forceinline__ void load_block(double (*dst)[PP], const double* A, i
   }
 }
 
-// 1 / d for 2^-1000 <= |d| <= 2^1000: the hardware's approximation, a
-// third-order and a second-order Newton step. Straight-line code, so that a
-// warp's reciprocals overlap its pivot search.
-__device__ __forceinline__ double newton_rcp(double d) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-  double e = fma(-d, x, 1.0);
-  x = fma(x, fma(e, e, e), x);
-  e = fma(-d, x, 1.0);
-  return fma(x, e, x);
-}
-
 // Inverses of the 16 x 16 triangles at logical rows and columns J0.. of D (row r
 // of it is row rowof(r) of D), column i per lane, by columns so that a step is
 // one FMA deep: the unit lower one to VL[q][k = column][row], the upper one to
