@@ -59,7 +59,6 @@ int consume_status(fp_ctx* c) {
   return FP_OK;
 }
 
-// Panel unit vectors of docs/src/elements/paneldefinition.md:15-35.
 int ensure_rhs(fp_ctx* c, int64_t k) {
   if (k <= c->cap_rhs) return FP_OK;
   dfree(c->d_rhs); dfree(c->d_x); dfree(c->d_r); dfree(c->d_w32); dfree(c->d_norms);

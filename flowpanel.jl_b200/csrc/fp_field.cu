@@ -113,8 +113,10 @@ k_uind_reduce(const double* __restrict__ partial, int nchunk, int64_t m, double*
 }
 
 // Panel chunks for m targets: enough blocks for sixteen per SM, so that the last
-// ones to finish are a small part, chunks of at least 512 panels, at most 16. In
-// FP32, where the chunks are part of the result, four per SM.
+// ones to finish are a small part, chunks of at least 512 panels, at most 16 (sources
+// too: the field of 4,455 panels at 30,000 targets 8.2 -> 7.5 ms, at 100,000 34.3 -> 23.9
+// against four per SM; up to 10,000 targets the same). In FP32, where the chunks are
+// part of the result, four per SM.
 int uind_chunks(int64_t m, int64_t n, bool fp32) {
   const int64_t blocks = (m + kFieldThreads - 1) / kFieldThreads;
   const int64_t want = (fp32 ? 4 : 16) * (int64_t)num_sms();

@@ -12,9 +12,10 @@
 // latency-bound), launched programmatically dependent. Nothing of it waits for
 // the host: the last kernel normalises V_{j+1} and leaves column j of the
 // Hessenberg matrix in mapped host memory, and the host, which only decides
-// when to stop, runs its rotations kAhead steps behind the launches. 252 steps at
-// N = 3,828 (A, 117 MB, about fills L2): 39 us a step, of which A v 23; with a
-// host synchronisation and plain loads a step took 236 us.
+// when to stop, runs its rotations kAhead steps behind the launches. N = 3,828 (A,
+// 117 MB, about fills L2): 38 us a step over 211 steps, of which A v 23 (41 over 350:
+// the passes over the basis grow); with a host synchronisation and plain loads 153.
+// 480 unknowns 87 -> 20 us a step, 12,000 320 -> 210.
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -114,7 +115,10 @@ k_sub_Vh(const double* V, int64_t ld, int nv, const double* h, double* w, int64_
 
 // parts of w = A v: 128 rows and one of kGemvSplitHost column ranges a CTA, 16
 // columns a stage; the first stages of A are under way before v is there
-constexpr int kMvRows = 128, kMvCols = 16, kMvStages = 3;   // four CTAs an SM: the grid of 3,828 rows in one wave
+// Three stages, four CTAs an SM. A step at 2,000, 3,828, 6,300, 8,000 and 12,000 unknowns
+// takes 23.5, 38.0, 81, 105 and 210 us; with two stages 23.8, 39.2, 71, 117 and 203, with
+// four (three CTAs) 23.8, 48.9, 80, 127 and 235.
+constexpr int kMvRows = 128, kMvCols = 16, kMvStages = 3;
 constexpr size_t kMvSmem = (size_t)kMvStages * kMvCols * (kMvRows + 1) * sizeof(double);
 __global__ void __launch_bounds__(kMvRows)
 k_matvec(const double* __restrict__ A, int64_t lda, int64_t n, const double* v, double* part) {

@@ -10,9 +10,9 @@
 // for latency: one CTA of 16 warps holds 64 rows of the panel in shared memory
 // for the whole panel, and blocks hand each other their factors through L2. One
 // launch per 64 columns, with the rows reloaded each time and SIMT products,
-// took 490 us a panel (strip and next-panel update included) where this takes
-// 240; factorisation of 480 unknowns 0.95 -> 0.60 ms, 1,840 3.47 -> 1.96,
-// 6,300 14.8 -> 8.5, 12,000 43.1 -> 33.4 ms.
+// took 490 us a panel (strip and next-panel update included) where k_panel64 takes
+// 141 and k_strip64 28 and 35 (captured, 3,500 rows); factorisation of 480 unknowns
+// 0.95 -> 0.49 ms, 1,840 3.47 -> 1.61, 6,300 16.7 -> 9.4, 12,000 58.9 -> 49.0.
 #include "fp_internal.cuh"
 
 namespace fpb {

@@ -493,7 +493,7 @@ k_pdiag(float* __restrict__ A, int64_t lda, int64_t n, int64_t k, float* __restr
 // next one's first (1,000 while most warps have work). The 32 x 32 inverses by
 // blocks of 8 (1.4 us; as one substitution of 32 steps 5 to 7). A block alone 25.2
 // -> 21.0 us, 18 of them in the kernel (27.3 -> 30.5 with a wait for each column
-// and those substitutions).
+// and those substitutions); 22.6 captured with the sums below.
 // The products that other warps' columns take off an entry are added up by themselves
 // and subtracted once: with up to 120 subtractions from an entry that may be much
 // larger than they are, a block's |A - LU| was twice that of the blocked kernel
