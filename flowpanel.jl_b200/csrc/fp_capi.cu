@@ -163,7 +163,8 @@ int fp_ctx_create(int device, fp_ctx** out) {
       cudaMalloc(&c->d_ticket, sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&c->d_p64, 8 * sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(c->d_p64, 0, 8 * sizeof(unsigned)) != cudaSuccess ||
-      cudaHostAlloc(&c->h_far, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+      cudaMalloc(&c->d_far, sizeof(unsigned)) != cudaSuccess ||
+      cudaMemset(c->d_far, 0, sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess || cudaMemset(c->d_ticket, 0, sizeof(unsigned)) != cudaSuccess) {
     delete c;
     return FP_ECUDA;
@@ -184,8 +185,7 @@ int fp_ctx_destroy(fp_ctx* c) {
   post_free(c);
   dfree(c->d_panels); dfree(c->d_src); dfree(c->d_tgt); dfree(c->d_wake);
   dfree(c->d_geo);
-  dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket); dfree(c->d_p64);
-  if (c->h_far) cudaFreeHost(c->h_far);
+  dfree(c->d_status); dfree(c->d_cert); dfree(c->d_ticket); dfree(c->d_p64); dfree(c->d_far);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t e : c->ktimer.pool) cudaEventDestroy(e);
@@ -239,10 +239,9 @@ int fp_set_geometry(fp_ctx* c, const double* nodes, int64_t nnodes, const int32_
     }
   }
   bool near_nodes = true;
-  for (int64_t i = 0; i < 3 * nnodes; ++i) {
+  for (int64_t i = 0; i < 3 * nnodes; ++i) near_nodes &= std::fabs(nodes[i]) < kNear;
+  for (int64_t i = 0; !near_nodes && i < 3 * nnodes; ++i)
     if (!std::isfinite(nodes[i])) return c->err.set(FP_EINVAL, "fp_set_geometry: non-finite node coordinate");
-    near_nodes = near_nodes && std::fabs(nodes[i]) < kNear;
-  }
   // device buffers only grow: a smaller body reuses them (leading dimension
   // unchanged), so a sequence of bodies allocates for the largest only
   if (npanels > c->capN) {

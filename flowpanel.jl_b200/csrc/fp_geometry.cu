@@ -31,7 +31,7 @@ __device__ __forceinline__ void store3(double* p, V3 a) { p[0] = a.x; p[1] = a.y
 
 __global__ void __launch_bounds__(128)
 k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* __restrict__ src, double* __restrict__ tgt,
-           int* __restrict__ far) {
+           unsigned* __restrict__ far, unsigned serial) {
   const int64_t p = (int64_t)blockIdx.x * 128 + threadIdx.x;
   if (p >= n) return;
   const int o0 = a.offsets[p], nn = a.offsets[p + 1] - o0;
@@ -103,7 +103,7 @@ k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* 
     cp = add(add(add(cc, scaled(t, __ddiv_rn(x, (double)nn))), scaled(o, __ddiv_rn(y, (double)nn))),
              scaled(nr, a.cp_offset ? a.cp_offset[p] : 1e-14));
   }
-  if (!near_point(cp.x, cp.y, cp.z)) *far = 1;   // also a NaN: a panel of no extent has no frame
+  if (!near_point(cp.x, cp.y, cp.z)) *far = serial;   // also a NaN: a panel of no extent has no frame
   tgt[p] = cp.x;
   tgt[n + p] = cp.y;
   tgt[2 * n + p] = cp.z;
@@ -115,12 +115,15 @@ k_geometry(GeometryArgs a, int64_t n, PanelRec* __restrict__ panels, SourceRec* 
 }  // namespace
 
 int launch_geometry(fp_ctx* c, const GeometryArgs& g) {
-  *c->h_far = 0;
-  k_geometry<<<(unsigned)((c->N + 127) / 128), 128, 0, c->stream>>>(g, c->N, c->d_panels, c->d_src, c->d_tgt, c->h_far);
+  ++c->geo_serial;
+  k_geometry<<<(unsigned)((c->N + 127) / 128), 128, 0, c->stream>>>(g, c->N, c->d_panels, c->d_src, c->d_tgt, c->d_far, c->geo_serial);
   ++c->nlaunch;
   FP_CUDA_TRY(c->err, cudaGetLastError());
-  FP_CUDA_TRY(c->err, cudaStreamSynchronize(c->stream));   // the caller may change its arrays (pinned ones too)
-  c->near_tgt = *c->h_far == 0;
+  // to pageable memory: done when it returns, and all before it in the stream with it,
+  // so that the caller may change its arrays (pinned ones too)
+  unsigned far = 0;
+  FP_CUDA_TRY(c->err, cudaMemcpyAsync(&far, c->d_far, sizeof(far), cudaMemcpyDeviceToHost, c->stream));
+  c->near_tgt = far != c->geo_serial;
   return FP_OK;
 }
 

@@ -76,7 +76,8 @@ struct fp_ctx {
   std::vector<double> h_tgt;            // 6 x N SoA copy of d_tgt, made when a call first needs it
   bool h_tgt_valid = false;
   bool near_nodes = true, near_tgt = true;   // every node, every control point is below kNear in size (fp_elements.cuh)
-  int* h_far = nullptr;                 // mapped host memory: a control point is not
+  unsigned* d_far = nullptr;            // serial of the last geometry with a control point that is not
+  unsigned geo_serial = 0;
 
   // device buffers
   fpb::PanelRec* d_panels = nullptr;    // N records
