@@ -12,7 +12,7 @@
 // launch per 64 columns, with the rows reloaded each time and SIMT products,
 // took 490 us a panel (strip and next-panel update included) where k_panel64 takes
 // 141 and k_strip64 28 and 35 (captured, 3,500 rows); factorisation of 480 unknowns
-// 0.95 -> 0.49 ms, 1,840 3.47 -> 1.61, 6,300 16.7 -> 9.4, 12,000 58.9 -> 49.0.
+// 0.95 -> 0.49 ms, 1,840 3.47 -> 1.65, 6,300 16.7 -> 9.5, 12,000 58.9 -> 49.1.
 #include "fp_internal.cuh"
 
 namespace fpb {
@@ -279,7 +279,10 @@ __device__ __forceinline__ void update(double (*C)[PP], double (*X)[PP], double 
 // X (64 columns of the panel, [column][row]) <- X U^-1 by 16-column sub-blocks:
 // U in Q ([column][k]), the inverses of its diagonal sub-blocks in VU. Eight
 // warps, an 8-row tile each, which depends on no other (no barriers). Returns
-// max|X|.
+// max|X|. A sub-block's solution by its inverse is refined once: without that its
+// error grows with the sub-block's condition, to 7e-14 of |L||U| where the rows of a
+// block differ by 1e6 in size and pivots are small (by substitution, and so, under
+// 1e-15). 480 unknowns 0.490 -> 0.494 ms, 1,840 1.626 -> 1.651, 6,300 9.47 -> 9.53.
 __device__ __forceinline__ double solve_l21(double (*X)[PP], double (*Q)[PP], const double* VU) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   if (warp >= 8) return 0.0;
@@ -297,28 +300,57 @@ __device__ __forceinline__ double solve_l21(double (*X)[PP], double (*Q)[PP], co
 #pragma unroll
         for (int h = 0; h < 2; ++h) dmma(d[h][i][0], d[h][i][1], a, Q[c + 8 * h + g][k + 4 * i + t]);
       }
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int e = 0; e < 2; ++e) X[c + 8 * h + 2 * t + e][row] -= d[h][0][e] + d[h][1][e];
-    __syncwarp();
-    double z[2][2][2] = {};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const double a = X[c + 4 * k + t][row];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) dmma(z[h][k & 1][0], z[h][k & 1][1], a, VU[q * VBLK + (8 * h + g) * VP + 4 * k + t]);
-    }
-    __syncwarp();
+    double b[2][2], x[2][2];   // the right-hand side and its solution
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const double v = z[h][0][e] + z[h][1][e];
-        X[c + 8 * h + 2 * t + e][row] = v;
-        mx = fmax(mx, fabs(v));
+        b[h][e] = X[c + 8 * h + 2 * t + e][row] - (d[h][0][e] + d[h][1][e]);
+        X[c + 8 * h + 2 * t + e][row] = b[h][e];
+        x[h][e] = 0.0;
       }
     __syncwarp();
+    // x = b inv(U), then once x += (b - x U) inv(U)
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+      double z[2][2][2] = {};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double a = X[c + 4 * k + t][row];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) dmma(z[h][k & 1][0], z[h][k & 1][1], a, VU[q * VBLK + (8 * h + g) * VP + 4 * k + t]);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          x[h][e] += z[h][0][e] + z[h][1][e];
+          X[c + 8 * h + 2 * t + e][row] = x[h][e];
+        }
+      __syncwarp();
+      if (pass == 1) break;
+      double u[2][2][2] = {};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double a = X[c + 4 * k + t][row];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const double w = 4 * k + t <= 8 * h + g ? Q[c + 8 * h + g][c + 4 * k + t] : 0.0;   // U alone: L lies below
+          dmma(u[h][k & 1][0], u[h][k & 1][1], a, w);
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) X[c + 8 * h + 2 * t + e][row] = b[h][e] - (u[h][0][e] + u[h][1][e]);
+      __syncwarp();
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) mx = fmax(mx, fabs(x[h][e]));
   }
   return mx;
 }
